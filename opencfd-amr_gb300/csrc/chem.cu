@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(kChemThreads) k_chem_advance(View<double> S, V
 // 0 and the component stride of each cell's FAB; state then species
 // components): one launch for every box, in the list's order.
 // ncell is bounded by *count when given (a list filled on the device); dtc gives
-// a step per cell when given.
+// a step per cell when given.  Without `off` the cells are 0 .. ncell - 1, without
+// `stride` the components are ncell apart (a contiguous array of cells).
 __global__ void __launch_bounds__(kChemThreads) k_chem_advance_list(const long long* __restrict__ off,
                                                                     const long long* __restrict__ stride,
                                                                     long long ncell, const unsigned* count,
@@ -182,8 +183,8 @@ __global__ void __launch_bounds__(kChemThreads) k_chem_advance_list(const long l
     if (count && c >= (long long)*count) return;
     if (c >= ncell) return;
     if (dtc) dt = dtc[c];
-    double* x = Ubuf + off[c];
-    const long long ns = stride[c];
+    double* x = Ubuf + (off ? off[c] : c);
+    const long long ns = stride ? stride[c] : ncell;
     double u[5], r[NSP];
 #pragma unroll
     for (int n = 0; n < 5; ++n) u[n] = x[n * ns];
@@ -261,12 +262,11 @@ __device__ __forceinline__ void cell_props(const double* x, long long ns, const 
     *rho_out = rho;
 }
 
-__global__ void k_chem_props(const long long* __restrict__ off, const long long* __restrict__ stride, long long ncell,
-                             const double* __restrict__ Ubuf, double* out, DevParm P) {
+__global__ void k_chem_props(long long ncell, const double* __restrict__ U, double* out, DevParm P) {
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncell;
          c += (long long)gridDim.x * blockDim.x) {
         double T, p, Y[NSP], rho, r[NSP];
-        cell_props(Ubuf + off[c], stride[c], P, &T, &p, Y, &rho, r);
+        cell_props(U + c, ncell, P, &T, &p, Y, &rho, r);
         out[c] = T;
         out[ncell + c] = p;
 #pragma unroll
@@ -338,8 +338,8 @@ struct SurThermo {
     float elem[3][NSP];   // atoms per unit mass (mol/kg) of each element
     double hw[NSP];       // d(rho e)/d(rho_n) of the chemistry update, -HP_n Ru / W_n (ChemAdvance.cpp:70-75)
 };
-constexpr int S_THERMO = (S_TOT + 15) / 16 * 16;
-constexpr int S_SUR_TOT = S_THERMO + (int)sizeof(SurThermo);
+__host__ __device__ constexpr int s_thermo(int ng) { return (s_tot(ng) + 15) / 16 * 16; }
+constexpr int s_sur_tot(int ng) { return s_thermo(ng) + (int)sizeof(SurThermo); }
 
 __device__ __forceinline__ void sur_thermo_build(SurThermo& th, double Ru) {
     const int n = threadIdx.x;
@@ -390,29 +390,32 @@ __device__ __forceinline__ float sur_temperature(const SurThermo& th, const floa
 }
 
 // One chemistry substep by the network for the cells of a list, 128 cells per
-// tile (thread t < 128 of the first warpgroup = cell t of the tile; all MLP_G
-// warpgroups share the network's epilogues): inputs (T, p, Y, log10 dt) ->
+// tile, NG tiles in flight per CTA (the first warpgroup of a tile's group has one
+// cell per thread; all 4 / NG warpgroups share the network's epilogues): inputs (T, p, Y, log10 dt) ->
 // rates of T and Y (the increments over the substep divided by dt).
 // Cells whose inputs leave the training range, or whose increments break the
 // species bounds or the H / O / N element balance beyond the guard's
 // tolerances, are appended to the fallback list for the FP64 substep.
 // Accepted cells update rho Y_n (clipped at 0) and rho E as the FP64 substep
 // does (ChemAdvance.cpp:62-80).
-__global__ void __launch_bounds__(128 * MLP_G) k_chem_surrogate(MlpNet net, const long long* __restrict__ off,
+template <int NG>
+__global__ void __launch_bounds__(MLP_THREADS) k_chem_surrogate(MlpNet net, const long long* __restrict__ off,
                                                         const long long* __restrict__ stride, long long ncell,
                                                         double* Ubuf, double dt, DevParm P, ocfd_surrogate_guard g,
                                                         long long* fb_off, long long* fb_stride, unsigned* fb_count,
                                                         unsigned long long* fb_total, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S_BAR);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S_BAR + 8);
-    SurThermo& th = *reinterpret_cast<SurThermo*>(sm + S_THERMO);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    constexpr int G = 4 / NG, GT = 128 * G;
+    const int warp = threadIdx.x >> 5, group = threadIdx.x / GT, tid = threadIdx.x % GT;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S_BAR) + group;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S_TSLOT);
+    unsigned char* a0 = sm + s_a0(group);
+    SurThermo& th = *reinterpret_cast<SurThermo*>(sm + s_thermo(NG));
     mlp_stage_weights(net, sm);
     sur_thermo_build(th, P.Ru);
     if (tid == 0) mbar_init(bar, 1);
     if (warp == 0) {
-        tmem_alloc(tslot, 128);
+        tmem_alloc(tslot, 128 * NG);
         tmem_relinquish();
     }
     fence_before_sync();
@@ -428,7 +431,7 @@ __global__ void __launch_bounds__(128 * MLP_G) k_chem_surrogate(MlpNet net, cons
     const float T_min = (float)g.T_min, T_max = (float)g.T_max, p_min = (float)g.p_min, p_max = (float)g.p_max;
     const float y_tol = (float)g.y_tol, elem_tol = (float)g.elem_tol;
     const float dy_rel = (float)g.dy_rel_max, y_floor = (float)g.y_floor;
-    for (long long t = blockIdx.x; t < ntile && ok; t += gridDim.x) {
+    for (long long t = blockIdx.x + gridDim.x * group; t < ntile && ok; t += gridDim.x * NG) {
         const long long c = t * 128 + tid;
         const bool valid = tid < 128 && c < ncell;
         double* x = nullptr;
@@ -436,8 +439,8 @@ __global__ void __launch_bounds__(128 * MLP_G) k_chem_surrogate(MlpNet net, cons
         double rho = 1.0, r[NSP];
         float Y[NSP], T = 0.0f, p = 1.0f;
         if (valid) {
-            x = Ubuf + off[c];
-            ns = stride[c];
+            x = Ubuf + (off ? off[c] : c);
+            ns = stride ? stride[c] : ncell;
             rho = dmax(x[0], P.smallr);
             const double rhoinv = 1.0 / rho;
             const double ux = x[ns] * rhoinv, uy = x[2 * ns] * rhoinv, uz = x[3 * ns] * rhoinv;
@@ -464,11 +467,15 @@ __global__ void __launch_bounds__(128 * MLP_G) k_chem_surrogate(MlpNet net, cons
         f[11] = (ldt - net.in_mu[11]) * net.in_isd[11];
         if (tid < 128) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
-                *reinterpret_cast<uint16_t*>(sm + S_A0 + kmajor_offset(tid, k, 128)) = k < MLP_IN ? bf16_bits(f[k]) : 0;
+            for (int k = MLP_IN; k < 16; ++k) f[k] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 16; k += 8)
+                *reinterpret_cast<uint4*>(a0 + kmajor_offset(tid, k, 128)) =
+                    make_uint4(bf16x2_bits(f[k], f[k + 1]), bf16x2_bits(f[k + 2], f[k + 3]),
+                               bf16x2_bits(f[k + 4], f[k + 5]), bf16x2_bits(f[k + 6], f[k + 7]));
         }
         float out[16];
-        ok = mlp_tile<MLP_G>(sm, tbase, bar, phase, out, nullptr, nullptr, 0);
+        ok = mlp_tile<G>(sm, a0, group, tid, tbase + 128 * group, bar, phase, out, nullptr, nullptr, 0);
         if (!ok || !valid) continue;
         float dY[NSP];
 #pragma unroll
@@ -545,15 +552,15 @@ __global__ void __launch_bounds__(128 * MLP_G) k_chem_surrogate(MlpNet net, cons
             x[4 * ns] += dei;
         } else {
             const unsigned q = atomicAdd(fb_count, 1u);
-            fb_off[q] = off[c];
-            fb_stride[q] = ns;
+            fb_off[q] = off ? off[c] : c;
+            if (fb_stride) fb_stride[q] = ns;
             atomicAdd(fb_total, 1ull);
         }
     }
     if (!ok && tid == 0) atomicOr(err, 1u);
     fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tbase, 128);
+    if (warp == 0) tmem_dealloc(tbase, 128 * NG);
 }
 
 ocfd_status launch_chem_surrogate(const ocfd_mlp* mlp, const long long* off, const long long* stride, long long ncell,
@@ -562,14 +569,21 @@ ocfd_status launch_chem_surrogate(const ocfd_mlp* mlp, const long long* off, con
                                   unsigned long long* fb_total, unsigned* err, int sms, cudaStream_t st) {
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(k_chem_surrogate, cudaFuncAttributeMaxDynamicSharedMemorySize, S_SUR_TOT) != cudaSuccess)
+        if (cudaFuncSetAttribute(k_chem_surrogate<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_sur_tot(1)) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_chem_surrogate<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_sur_tot(2)) !=
+                cudaSuccess)
             return check_launch("surrogate attribute");
         configured = true;
     }
     if (ncell <= 0) return OCFD_OK;
     const long long ntile = (ncell + 127) / 128;
-    k_chem_surrogate<<<(unsigned)std::min<long long>(ntile, sms), 128 * MLP_G, S_SUR_TOT, st>>>(
-        mlp_net(mlp), off, stride, ncell, U, dt, P, g, fb_off, fb_stride, fb_count, fb_total, err);
+    if (mlp_groups(ntile, sms) == 2)
+        k_chem_surrogate<2><<<(unsigned)sms, MLP_THREADS, s_sur_tot(2), st>>>(
+            mlp_net(mlp), off, stride, ncell, U, dt, P, g, fb_off, fb_stride, fb_count, fb_total, err);
+    else
+        k_chem_surrogate<1><<<(unsigned)ntile, MLP_THREADS, s_sur_tot(1), st>>>(
+            mlp_net(mlp), off, stride, ncell, U, dt, P, g, fb_off, fb_stride, fb_count, fb_total, err);
     return check_launch("surrogate chemistry substep");
 }
 
@@ -1294,43 +1308,12 @@ extern "C" ocfd_status ocfd_rhs_chem_eb_box_f64(ocfd_context* ctx, const ocfd_ar
 }
 
 // ------------------------------------------------------------ 0D cells
-namespace ocfd {
-__global__ void k_iota_cells(long long* off, long long* stride, long long n) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        off[c] = c;
-        stride[c] = n;
-    }
-}
-
-struct CellList {
-    long long* off = nullptr;
-    long long* stride = nullptr;
-    ~CellList() {
-        cudaFree(off);
-        cudaFree(stride);
-    }
-    bool make(long long n, int sms, cudaStream_t st) {
-        if (cudaMalloc(&off, sizeof(long long) * n) != cudaSuccess ||
-            cudaMalloc(&stride, sizeof(long long) * n) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        long long b = (n + 255) / 256;
-        if (b > (long long)sms * 16) b = (long long)sms * 16;
-        k_iota_cells<<<(int)b, 256, 0, st>>>(off, stride, n);
-        return true;
-    }
-};
-}  // namespace ocfd
-
 extern "C" ocfd_status ocfd_chem_cells_advance(ocfd_context* ctx, int64_t n, double* U, const double* dt_cells,
                                                double dt, void* stream) {
     using namespace ocfd;
     if (!ctx || n <= 0 || !U) return fail(OCFD_BAD_ARG, "ocfd_chem_cells_advance");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    CellList L;
-    if (!L.make(n, ctx->num_sms, st)) return fail(OCFD_OUT_OF_MEMORY, "ocfd_chem_cells_advance");
-    ocfd_status s = launch_chem_advance_list(L.off, L.stride, n, U, dt, ctx->parm, st, nullptr, dt_cells);
+    ocfd_status s = launch_chem_advance_list(nullptr, nullptr, n, U, dt, ctx->parm, st, nullptr, dt_cells);
     if (cudaStreamSynchronize(st) != cudaSuccess) return check_launch("ocfd_chem_cells_advance");
     return s;
 }
@@ -1340,11 +1323,9 @@ extern "C" ocfd_status ocfd_chem_cells_props(ocfd_context* ctx, int64_t n, const
     using namespace ocfd;
     if (!ctx || n <= 0 || !U || !out) return fail(OCFD_BAD_ARG, "ocfd_chem_cells_props");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    CellList L;
-    if (!L.make(n, ctx->num_sms, st)) return fail(OCFD_OUT_OF_MEMORY, "ocfd_chem_cells_props");
     long long b = (n + 127) / 128;
     if (b > (long long)ctx->num_sms * 32) b = (long long)ctx->num_sms * 32;
-    k_chem_props<<<(int)b, 128, 0, st>>>(L.off, L.stride, n, U, out, ctx->parm);
+    k_chem_props<<<(int)b, 128, 0, st>>>(n, U, out, ctx->parm);
     ocfd_status s = check_launch("ocfd_chem_cells_props");
     if (cudaStreamSynchronize(st) != cudaSuccess) return check_launch("ocfd_chem_cells_props");
     return s;
@@ -1369,29 +1350,23 @@ extern "C" ocfd_status ocfd_chem_cells_surrogate(ocfd_context* ctx, ocfd_mlp* ml
     using namespace ocfd;
     if (!ctx || !mlp || !g || n <= 0 || !U) return fail(OCFD_BAD_ARG, "ocfd_chem_cells_surrogate");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    CellList L, F;
-    unsigned* cnt = nullptr;
-    unsigned long long* tot = nullptr;
-    if (!L.make(n, ctx->num_sms, st) || !F.make(n, ctx->num_sms, st) || cudaMalloc(&cnt, sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc(&tot, sizeof(unsigned long long)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(cnt);
-        return fail(OCFD_OUT_OF_MEMORY, "ocfd_chem_cells_surrogate");
-    }
-    cudaMemsetAsync(cnt, 0, sizeof(unsigned), st);
-    cudaMemsetAsync(tot, 0, sizeof(unsigned long long), st);
+    // fallback counters and list (the cells' indices; a component stride of n) in
+    // the context's scratch pool
+    unsigned long long* tot = static_cast<unsigned long long*>(scratch(ctx, 16 + sizeof(long long) * (size_t)n));
+    if (!tot) return fail(OCFD_OUT_OF_MEMORY, "ocfd_chem_cells_surrogate");
+    unsigned* cnt = reinterpret_cast<unsigned*>(tot + 1);
+    long long* list = reinterpret_cast<long long*>(tot + 2);
+    cudaMemsetAsync(tot, 0, 16, st);
     cudaMemsetAsync(ctx->d_error, 0, sizeof(uint32_t), st);
-    ocfd_status s = launch_chem_surrogate(mlp, L.off, L.stride, n, U, dt, ctx->parm, *g, F.off, F.stride, cnt, tot,
+    ocfd_status s = launch_chem_surrogate(mlp, nullptr, nullptr, n, U, dt, ctx->parm, *g, list, nullptr, cnt, tot,
                                           ctx->d_error, ctx->num_sms, st);
-    if (s == OCFD_OK) s = launch_chem_advance_list(F.off, F.stride, n, U, dt, ctx->parm, st, cnt, nullptr);
+    if (s == OCFD_OK) s = launch_chem_advance_list(list, nullptr, n, U, dt, ctx->parm, st, cnt, nullptr);
     unsigned long long h = 0;
     uint32_t e = 0;
     if (cudaMemcpyAsync(&h, tot, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(&e, ctx->d_error, sizeof(e), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         s = check_launch("ocfd_chem_cells_surrogate");
-    cudaFree(cnt);
-    cudaFree(tot);
     if (s == OCFD_OK && e) s = fail(OCFD_TIMEOUT, "ocfd_chem_cells_surrogate: a tensor-core completion wait ran out");
     if (fallbacks) *fallbacks = (int64_t)h;
     return s;

@@ -66,18 +66,22 @@ __global__ void __launch_bounds__(128) k_tc_gemm(const uint16_t* __restrict__ A,
 }
 
 // Training forward: X [M x 16] BF16 normalised inputs (row-major) -> Y [M x 16]
-// FP32, stashing Z_l, H_l (l = 1..4) as [4][M/128][128 x 128] blocks; MLP_G
-// warpgroups per 128-row tile (the first stages the inputs and writes Y).
-__global__ void __launch_bounds__(128 * MLP_G) k_mlp_forward(MlpNet net, const uint16_t* __restrict__ X, float* Y,
+// FP32, stashing Z_l, H_l (l = 1..4) as [4][M/128][128 x 128] blocks; NG tiles in
+// flight per CTA, 4 / NG warpgroups per tile (the first stages the inputs and
+// writes Y).
+template <int NG>
+__global__ void __launch_bounds__(MLP_THREADS) k_mlp_forward(MlpNet net, const uint16_t* __restrict__ X, float* Y,
                                                              float* Z, uint16_t* H, int ntile, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S_BAR);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S_BAR + 8);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    constexpr int G = 4 / NG, GT = 128 * G;
+    const int tid = threadIdx.x, warp = tid >> 5, group = tid / GT, gt = tid % GT;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S_BAR) + group;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S_TSLOT);
+    unsigned char* a0 = sm + s_a0(group);
     mlp_stage_weights(net, sm);
-    if (tid == 0) mbar_init(bar, 1);
+    if (gt == 0) mbar_init(bar, 1);
     if (warp == 0) {
-        tmem_alloc(tslot, 128);
+        tmem_alloc(tslot, 128 * NG);
         tmem_relinquish();
     }
     fence_before_sync();
@@ -86,26 +90,28 @@ __global__ void __launch_bounds__(128 * MLP_G) k_mlp_forward(MlpNet net, const u
     const uint32_t tbase = *tslot;
     uint32_t phase = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < ntile && ok; t += gridDim.x) {
-        const long long row = (long long)t * 128 + tid;
-        if (tid < 128) {
+    for (int t = blockIdx.x + gridDim.x * group; t < ntile && ok; t += gridDim.x * NG) {
+        const long long row = (long long)t * 128 + gt;
+        if (gt < 128) {
             // one row of 16 BF16 inputs: two 16-byte core-matrix rows
             const uint4* xr = reinterpret_cast<const uint4*>(X + row * 16);
-            *reinterpret_cast<uint4*>(sm + S_A0 + kmajor_offset(tid, 0, 128)) = xr[0];
-            *reinterpret_cast<uint4*>(sm + S_A0 + kmajor_offset(tid, 8, 128)) = xr[1];
+            *reinterpret_cast<uint4*>(a0 + kmajor_offset(gt, 0, 128)) = xr[0];
+            *reinterpret_cast<uint4*>(a0 + kmajor_offset(gt, 8, 128)) = xr[1];
         }
         float out[16];
         // stash layout: block t of layer l at ((l * ntile + t) * 128 + row) * 128
-        ok = mlp_tile<MLP_G>(sm, tbase, bar, phase, out, Z ? Z + (long long)t * 128 * 128 : nullptr,
-                             H ? H + (long long)t * 128 * 128 : nullptr, (long long)ntile * 128);
-        if (ok && tid < 128)
+        ok = mlp_tile<G>(sm, a0, group, gt, tbase + 128 * group, bar, phase, out,
+                         Z ? Z + (long long)t * 128 * 128 : nullptr, H ? H + (long long)t * 128 * 128 : nullptr,
+                         (long long)ntile * 128);
+        if (ok && gt < 128)
 #pragma unroll
-            for (int i = 0; i < 16; ++i) Y[row * 16 + i] = out[i];
+            for (int i = 0; i < 16; i += 4)
+                *reinterpret_cast<float4*>(Y + row * 16 + i) = make_float4(out[i], out[i + 1], out[i + 2], out[i + 3]);
     }
-    if (!ok && tid == 0) atomicOr(err, 1u);
+    if (!ok && gt == 0) atomicOr(err, 1u);
     fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tbase, 128);
+    if (warp == 0) tmem_dealloc(tbase, 128 * NG);
 }
 
 __device__ __forceinline__ float gelu_grad(float z) {
@@ -371,7 +377,8 @@ MlpNet mlp_net(const ocfd_mlp* n) {
 static ocfd_status mlp_configure() {
     static bool done = false;
     if (done) return OCFD_OK;
-    if (cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, S_TOT) != cudaSuccess ||
+    if (cudaFuncSetAttribute(k_mlp_forward<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_tot(1)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_mlp_forward<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_tot(2)) != cudaSuccess ||
         cudaFuncSetAttribute(k_mlp_bwd_data, cudaFuncAttributeMaxDynamicSharedMemorySize, SD_TOT) != cudaSuccess ||
         cudaFuncSetAttribute(k_mlp_bwd_weight, cudaFuncAttributeMaxDynamicSharedMemorySize, SW_TOT) != cudaSuccess)
         return check_launch("MLP kernel attributes");
@@ -384,8 +391,11 @@ static ocfd_status mlp_forward(ocfd_mlp* n, const float* X, long long M, cudaStr
     const int sms = n->ctx->num_sms;
     k_mlp_pack<<<grid_for(M * 16, 256, sms), 256, 0, st>>>(X, n->Xb, M);
     const int ntile = (int)(M / 128);
-    k_mlp_forward<<<std::min(ntile, sms), 128 * MLP_G, S_TOT, st>>>(net_of(n), n->Xb, n->Y, n->Z, n->H, ntile,
-                                                                    n->ctx->d_error);
+    if (mlp_groups(ntile, sms) == 2)
+        k_mlp_forward<2><<<sms, MLP_THREADS, s_tot(2), st>>>(net_of(n), n->Xb, n->Y, n->Z, n->H, ntile, n->ctx->d_error);
+    else
+        k_mlp_forward<1><<<ntile, MLP_THREADS, s_tot(1), st>>>(net_of(n), n->Xb, n->Y, n->Z, n->H, ntile,
+                                                               n->ctx->d_error);
     return check_launch("MLP forward");
 }
 

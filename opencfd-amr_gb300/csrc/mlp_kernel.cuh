@@ -38,13 +38,16 @@ __host__ __device__ constexpr int WOFF(int l) { return l == 0 ? 0 : 2048 + (l - 
 constexpr int WTOT = 53248;
 __host__ __device__ constexpr int BOFF(int l) { return 128 * l; }
 constexpr int BTOT = 528;
-// shared memory of the fused kernel (bytes)
-constexpr int S_W = 0;                        // the five B operands, K-major, as WOFF * 2
-constexpr int S_A0 = WTOT * 2;                // 128 x 16 input operand
-constexpr int S_H = S_A0 + 128 * 16 * 2;      // 128 x 128 hidden operand
-constexpr int S_B = S_H + 128 * 128 * 2;      // biases, FP32
-constexpr int S_BAR = S_B + BTOT * 4;
-constexpr int S_TOT = S_BAR + 16;
+// shared memory of the fused kernel with NG tiles in flight (bytes): the weights
+// and biases once, each tile's operands and completion barrier
+constexpr int S_W = 0;             // the five B operands, K-major, as WOFF * 2
+constexpr int S_B = WTOT * 2;      // biases, FP32
+constexpr int S_BAR = S_B + BTOT * 4;  // two barriers, then the TMEM base
+constexpr int S_TSLOT = S_BAR + 16;
+constexpr int S_OP = (S_TSLOT + 16 + 127) / 128 * 128;
+constexpr int S_A0_BYTES = 128 * 16 * 2, S_H_BYTES = 128 * 128 * 2;  // input and hidden operand of a tile
+__host__ __device__ constexpr int s_a0(int g) { return S_OP + g * (S_A0_BYTES + S_H_BYTES); }
+__host__ __device__ constexpr int s_tot(int ng) { return s_a0(ng); }
 
 struct MlpNet {
     const uint16_t* W;  // BF16 weights, WTOT elements
@@ -74,35 +77,57 @@ __device__ __forceinline__ void mlp_stage_weights(const MlpNet& net, unsigned ch
     for (int e = threadIdx.x; e < BTOT; e += blockDim.x) sb[e] = net.b[e];
 }
 
-// warpgroups (of 128 threads) that share one 128-row tile: the bias + GELU
-// epilogue of a hidden layer (128 columns per row, erf and BF16 packing per
-// element) takes far longer than the layer's MMAs, so it is split over MLP_G
-// warpgroups by columns
-constexpr int MLP_G = 4;
+// Threads of a CTA: 512, as NG groups of G warpgroups (128 threads each).  A group
+// takes one 128-row tile through the network; the bias + GELU epilogue of a hidden
+// layer (erf and BF16 packing per element) takes far longer than the layer's MMAs,
+// so it is split over the group's G warpgroups by columns.  With NG = 2 the two
+// tiles' waits (MMA completion, barriers, the 128-thread prologue and tail)
+// overlap the other tile's epilogue; with fewer tiles than SMs one tile per CTA on
+// all four warpgroups has the shorter latency.  mlp_groups() draws the line.
+// Measured with one tile -> two tiles in flight and the packed BF16 conversion,
+// same bits: one surrogate substep of 2^20 cells, a quarter of them falling back
+// to FP64, 4.55 -> 3.63 ms (this and the cell lists no longer made for
+// contiguous cells); a training step of 8192 rows (64 tiles) 528 -> 508 us.
+constexpr int MLP_THREADS = 512;
+inline int mlp_groups(long long ntile, int sms) { return ntile > sms ? 2 : 1; }
 
-// one 128-row tile through the five layers; the input operand (S_A0) is staged.
-// The CTA has 128 G threads: thread t serves row t % 128 (warp w reads TMEM
-// lanes 32 (w % 4) .. 32 (w % 4) + 31) and columns [(t / 128) 128 / G,
-// (t / 128 + 1) 128 / G) of every hidden layer; the output layer's 16 columns go
-// to the first warpgroup (out[]).  Hidden activations go to `zs` / `hs` (FP32
-// pre-activations, BF16 activations; may be null).  Returns false when an MMA
-// completion wait ran out.
+// two floats to packed BF16, round to nearest even (lo in the low half)
+__device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
+// barrier of one group of a CTA (whole warps; id 0 is __syncthreads')
+__device__ __forceinline__ void group_sync(int group, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(threads) : "memory");
+}
+
+// one 128-row tile through the five layers; the input operand (a0, followed by the
+// hidden operand) is staged.  Called by a group's 128 G threads: thread gt serves
+// row gt % 128 (warp w reads TMEM lanes 32 (w % 4) .. 32 (w % 4) + 31) and columns
+// [(gt / 128) 128 / G, (gt / 128 + 1) 128 / G) of every hidden layer; the output
+// layer's 16 columns go to the first warpgroup (out[]).  Hidden activations go to
+// `zs` / `hs` (FP32 pre-activations, BF16 activations; may be null).  Returns
+// false when an MMA completion wait ran out.
 template <int G>
-__device__ __forceinline__ bool mlp_tile(unsigned char* sm, uint32_t tbase, uint64_t* bar, uint32_t& phase,
-                                         float* out, float* zs, uint16_t* hs, long long ld) {
-    static_assert(G == 1 || G == 2 || G == 4, "warpgroups per tile");
+__device__ __forceinline__ bool mlp_tile(unsigned char* sm, unsigned char* a0, int group, int gt, uint32_t tbase,
+                                         uint64_t* bar, uint32_t& phase, float* out, float* zs, uint16_t* hs,
+                                         long long ld) {
+    static_assert(G == 2 || G == 4, "warpgroups per tile");
     constexpr int CW = MLP_H / G;
-    const int tid = threadIdx.x, row = tid & 127, cg = tid >> 7;
+    const int row = gt & 127, cg = gt >> 7;
     const float* sb = reinterpret_cast<const float*>(sm + S_B);
-    const uint32_t trow = tbase + ((uint32_t)(((tid >> 5) & 3) * 32) << 16);
+    unsigned char* h = a0 + S_A0_BYTES;
+    const uint32_t trow = tbase + ((uint32_t)(((gt >> 5) & 3) * 32) << 16);
     for (int l = 0; l < 5; ++l) {
         fence_async_smem();
         fence_before_sync();
-        __syncthreads();
+        group_sync(group, 128 * G);
         fence_after_sync();
-        if (tid == 0) {
+        if (gt == 0) {
             const uint32_t idesc = idesc_bf16_f32(128, LN(l));
-            const unsigned char* A = sm + (l == 0 ? S_A0 : S_H);
+            const unsigned char* A = l == 0 ? a0 : h;
             const unsigned char* B = sm + S_W + WOFF(l) * 2;
             for (int ks = 0; ks < LK(l) / 16; ++ks)
                 mma_bf16(tbase, smem_desc(smem_u32(A + ks * 128 * 32)), smem_desc(smem_u32(B + ks * LN(l) * 32)),
@@ -123,18 +148,17 @@ __device__ __forceinline__ bool mlp_tile(unsigned char* sm, uint32_t tbase, uint
                 for (int q = 0; q < 4; ++q) {
                     uint32_t pk[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int i = q * 8 + e * 2;
-                        const float z0 = v[i] + sb[BOFF(l) + c0 + i], z1 = v[i + 1] + sb[BOFF(l) + c0 + i + 1];
-                        pk[e] = (uint32_t)bf16_bits(gelu(z0)) | ((uint32_t)bf16_bits(gelu(z1)) << 16);
-                        if (zs) {
-                            float* zr = zs + (long long)l * 128 * ld + (long long)row * 128 + c0 + i;
-                            zr[0] = z0;
-                            zr[1] = z1;
-                        }
+                    for (int e = 0; e < 2; ++e) {
+                        const int i = q * 8 + e * 4;
+                        const float4 b = *reinterpret_cast<const float4*>(sb + BOFF(l) + c0 + i);
+                        const float4 z = make_float4(v[i] + b.x, v[i + 1] + b.y, v[i + 2] + b.z, v[i + 3] + b.w);
+                        pk[2 * e] = bf16x2_bits(gelu(z.x), gelu(z.y));
+                        pk[2 * e + 1] = bf16x2_bits(gelu(z.z), gelu(z.w));
+                        if (zs)
+                            *reinterpret_cast<float4*>(zs + (long long)l * 128 * ld + (long long)row * 128 + c0 + i) = z;
                     }
                     const uint4 w = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    *reinterpret_cast<uint4*>(sm + S_H + kmajor_offset(row, c0 + q * 8, 128)) = w;
+                    *reinterpret_cast<uint4*>(h + kmajor_offset(row, c0 + q * 8, 128)) = w;
                     if (hs)
                         *reinterpret_cast<uint4*>(hs + (long long)l * 128 * ld + (long long)row * 128 + c0 + q * 8) = w;
                 }
