@@ -54,7 +54,14 @@ ocfd_status mech_upload(const ocfd_parm& p) {
         }
     for (int a = 0; a < NSP; ++a) {
         md.inv_mw[a] = 1.0 / t.mw[a];
-        for (int b = 0; b < NSP; ++b) md.wratio[a][b] = t.mw[a] / t.mw[b];
+        md.hw[a] = -t.HP[a] * p.Ru * md.inv_mw[a];
+        md.a0w[a] = t.A0[a] * md.inv_mw[a];
+        for (int k = 0; k < 5; ++k) md.nw[k][a] = k * t.mw[a];
+        for (int h = 0; h < 2; ++h) {
+            const double* c = h ? t.hi[a] : t.lo[a];
+            const double u[6] = {c[0] - 1.0, c[1] / 2.0, c[2] / 3.0, c[3] / 4.0, c[4] / 5.0, h ? c[5] - t.lo[a][5] : 0.0};
+            for (int k = 0; k < 6; ++k) md.uw[h][k][a] = u[k] * md.inv_mw[a];
+        }
         // speciesInternalEnergy (LiDryer.H:531-614) at 250 K (low range) and 3500 K (high range)
         auto ums = [&](double T, int hi) {
             const double* c = hi ? t.hi[a] : t.lo[a];
@@ -66,6 +73,20 @@ ocfd_status mech_upload(const ocfd_parm& p) {
         md.umin_w[a] = ums(250.0, 0) * md.inv_mw[a];
         md.umax_w[a] = ums(3500.0, 1) * md.inv_mw[a];
     }
+    // H and O atoms of H2O, H, O, OH, HO2, H2O2
+    const double nh[NSP - 3] = {2, 1, 0, 1, 1, 2}, no[NSP - 3] = {1, 0, 1, 1, 2, 2};
+    for (int h = 0; h < 2; ++h)
+        for (int n = 0; n < NSP - 3; ++n) {
+            const auto* tab = h ? t.hi : t.lo;
+            double a[7];
+            for (int k = 0; k < 7; ++k) a[k] = tab[n + 2][k] - 0.5 * nh[n] * tab[0][k] - 0.5 * no[n] * tab[1][k];
+            // gibbs, LiDryer.H:70-154: a0 (1 - lnT) - a1/2 T - a2/6 T^2 - a3/12 T^3 - a4/20 T^4 + a5/T - a6
+            const double g[7] = {a[0] - a[6], -a[1] / 2.0, -a[2] / 6.0, -a[3] / 12.0, -a[4] / 20.0, a[5], -a[0]};
+            for (int k = 0; k < 7; ++k) md.gp[h][n][k] = g[k];
+        }
+    md.inv_ru = 1.0 / p.Ru;
+    md.rs = p.Ru / p.Patm * 1e6;
+    md.inv_rs = 1.0 / md.rs;
     if (cudaMemcpyToSymbol(c_mder, &md, sizeof(md)) != cudaSuccess) {
         cudaError_t e = cudaGetLastError();
         return fail(OCFD_LAUNCH_FAIL, std::string("mechanism upload: ") + cudaGetErrorString(e));
@@ -94,39 +115,28 @@ ocfd_status mech_upload(const ocfd_parm& p) {
 // One semi-implicit chemistry substep of one cell, in place: the lambda of
 // EBR::chemical_advance, Source/CHEM/ChemAdvance.cpp:27-82.  u = rho, mx, my,
 // mz, E (E updated), r = the 9 partial densities (updated).
-__device__ __forceinline__ void chem_cell(const double* u, double& E, double* r, double dt, const DevParm& P,
-                                          const SmemMat& U) {
+__device__ __forceinline__ void chem_cell(const double* u, double& E, double* r, double dt, const DevParm& P) {
     const double rho = dmax(u[0], P.smallr);
-    const double rhoinv = 1.0 / rho;
+    const double rhoinv = rcp_nr(rho);
     const double ux = u[1] * rhoinv, uy = u[2] * rhoinv, uz = u[3] * rhoinv;
-    const double kineng = 0.5 * (ux * ux + uy * uy + uz * uz);
-    const double ei = E - rho * kineng;
-    double cc[NSP], wdot[NSP], drho[NSP];
+    const double ei = fma(-0.5, fma(u[3], uz, fma(u[2], uy, u[1] * ux)), E);
+    double cc[NSP], drho[NRE];
     const double T = get_t_given_ey(ei, r, P.Ru);
+    double mixture = 0.0;
 #pragma unroll
-    for (int n = 0; n < NSP; n++) cc[n] = r[n] * c_mder.inv_mw[n] * 1e-6;
-    for (int a = 0; a < NSP; ++a)
-        for (int b = 0; b < NSP; ++b) U(a, b) = 0.0;
-    production_rate(wdot, U, cc, T, P.Ru, P.Patm);
-    for (int a = 0; a < NSP; ++a) {
-        for (int b = 0; b < NSP; ++b) {
-            const double ar = U(a, b);
-            double v = (a == b ? 1.0 : 0.0);
-            v -= ar * c_mder.wratio[a][b] * dt;
-            U(a, b) = v;
-        }
-        U(a, NSP) = wdot[a] * c_mech.mw[a] * 1e6 * dt;
+    for (int n = 0; n < NSP; n++) {
+        cc[n] = r[n] * c_mder.inv_mw[n] * 1e-6;
+        mixture += cc[n];
     }
-    gauss_solve(U, drho);
+    chem_increment(cc, mixture, T, dt, drho);
     double dei = 0;
 #pragma unroll
-    for (int n = 0; n < NSP; ++n) {
-        double v = r[n] + drho[n];
-        if (v < 0) v = 0.0;
-        r[n] = v;
+    for (int n = 0; n < NRE; ++n) {
+        const double v = r[n] + drho[n];
+        r[n] = v < 0 ? 0.0 : v;
+        dei = fma(c_mder.hw[n], drho[n], dei);
     }
-#pragma unroll
-    for (int n = 0; n < NSP; ++n) dei += -c_mech.HP[n] * P.Ru * c_mder.inv_mw[n] * drho[n];
+    if (r[NSP - 1] < 0) r[NSP - 1] = 0.0;  // N2: no increment, clipped as the others
     E += dei;
 }
 
@@ -147,8 +157,6 @@ __device__ __forceinline__ void renorm_cell(double rho, double* r) {
 
 __global__ void __launch_bounds__(kChemThreads) k_chem_advance(View<double> S, View<double> sp, CellBox B,
                                                                double dt, DevParm P, int renorm) {
-    extern __shared__ double smem[];
-    const SmemMat U{smem + threadIdx.x, (int)blockDim.x};
     const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (c >= B.count()) return;
     int i, j, k;
@@ -159,7 +167,7 @@ __global__ void __launch_bounds__(kChemThreads) k_chem_advance(View<double> S, V
 #pragma unroll
     for (int n = 0; n < NSP; ++n) r[n] = sp(i, j, k, n);
     double E = u[4];
-    chem_cell(u, E, r, dt, P, U);
+    chem_cell(u, E, r, dt, P);
     if (renorm) renorm_cell(u[0], r);
 #pragma unroll
     for (int n = 0; n < NSP; ++n) sp(i, j, k, n) = r[n];
@@ -177,8 +185,6 @@ __global__ void __launch_bounds__(kChemThreads) k_chem_advance_list(const long l
                                                                     long long ncell, const unsigned* count,
                                                                     const double* __restrict__ dtc, double* Ubuf,
                                                                     double dt, DevParm P, int renorm) {
-    extern __shared__ double smem[];
-    const SmemMat U{smem + threadIdx.x, (int)blockDim.x};
     const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (count && c >= (long long)*count) return;
     if (c >= ncell) return;
@@ -191,7 +197,7 @@ __global__ void __launch_bounds__(kChemThreads) k_chem_advance_list(const long l
 #pragma unroll
     for (int n = 0; n < NSP; ++n) r[n] = x[(5 + n) * ns];
     double E = u[4];
-    chem_cell(u, E, r, dt, P, U);
+    chem_cell(u, E, r, dt, P);
     if (renorm) renorm_cell(u[0], r);
 #pragma unroll
     for (int n = 0; n < NSP; ++n) x[(5 + n) * ns] = r[n];
@@ -217,20 +223,11 @@ __global__ void k_spec_renorm(View<const double> S, View<double> sp, CellBox B) 
     }
 }
 
-ocfd_status configure_chem() {
-    if (cudaFuncSetAttribute(k_chem_advance, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(double) * 90 * kChemThreads)) != cudaSuccess ||
-        cudaFuncSetAttribute(k_chem_advance_list, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(double) * 90 * kChemThreads)) != cudaSuccess)
-        return check_launch("configure_chem");
-    return OCFD_OK;
-}
-
 ocfd_status launch_chem_advance(View<double> S, View<double> sp, const CellBox& B, double dt, const DevParm& P,
                                 cudaStream_t st, bool renorm) {
     const long long n = (long long)B.n[0] * B.n[1] * B.n[2];
     const int blocks = (int)((n + kChemThreads - 1) / kChemThreads);
-    k_chem_advance<<<blocks, kChemThreads, sizeof(double) * 90 * kChemThreads, st>>>(S, sp, B, dt, P, renorm ? 1 : 0);
+    k_chem_advance<<<blocks, kChemThreads, 0, st>>>(S, sp, B, dt, P, renorm ? 1 : 0);
     return check_launch("chemistry substep");
 }
 
@@ -239,7 +236,7 @@ ocfd_status launch_chem_advance_list(const long long* off, const long long* stri
                                      const double* dtc, bool renorm) {
     if (ncell <= 0) return OCFD_OK;
     const long long blocks = (ncell + kChemThreads - 1) / kChemThreads;
-    k_chem_advance_list<<<(unsigned)blocks, kChemThreads, sizeof(double) * 90 * kChemThreads, st>>>(
+    k_chem_advance_list<<<(unsigned)blocks, kChemThreads, 0, st>>>(
         off, stride, ncell, count, dtc, U, dt, P, renorm ? 1 : 0);
     return check_launch("chemistry substep (cell list)");
 }

@@ -11,14 +11,6 @@ namespace ocfd {
 
 constexpr int kChemThreads = 128;
 
-// Per-thread 9x10 matrix in shared memory, element-major so that the threads
-// of a warp touch consecutive words.
-struct SmemMat {
-    double* base;
-    int stride;
-    __device__ __forceinline__ double& operator()(int r, int c) const { return base[(r * 10 + c) * stride]; }
-};
-
 struct CellBox {
     int lo[3], n[3];
     __host__ __device__ __forceinline__ long long count() const { return (long long)n[0] * n[1] * n[2]; }

@@ -12,7 +12,6 @@
 
 namespace ocfd {
 
-ocfd_status configure_chem();
 
 static thread_local std::string g_last_error;
 
@@ -164,7 +163,6 @@ ocfd_status ocfd_context_create(const ocfd_parm* parm, int device, ocfd_context*
     ocfd_status s = mech_upload(*parm);
     if (s == OCFD_OK) s = configure_rhs_regular();
     if (s == OCFD_OK) s = configure_rhs_regular_f32();
-    if (s == OCFD_OK) s = configure_chem();
     if (s == OCFD_OK) s = configure_eb_tile();
     if (s == OCFD_OK) s = eb_static_scratch_resolve(ctx);
     if (s != OCFD_OK) {
