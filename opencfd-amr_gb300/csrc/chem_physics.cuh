@@ -127,14 +127,33 @@ __device__ __forceinline__ void ckytx(const double* y, double* x) {
     for (int i = 0; i < NSP; ++i) x[i] = y[i] / c_mech.mw[i] * YOWINV;
 }
 
+// The Newton loop of GET_T_GIVEN_EY (LiDryer.H:833-888) in the reference's
+// operation order, from the starting value t1
+__device__ __forceinline__ double newton_reference_order(double ein, const double* rhoi, double Ru, double t1) {
+    for (int i = 0; i < 200; ++i) {
+        const double e1 = ckubms(t1, rhoi, Ru);
+        const double cv = ckcvbs(t1, rhoi, Ru);
+        double dt = (ein - e1) / cv;
+        if (dt > 100.0) dt = 100.0;
+        else if (dt < -100.0) dt = -100.0;
+        else if (fabs(dt) < 1e-7) break;
+        else if (t1 + dt == t1) break;
+        t1 += dt;
+    }
+    return t1;
+}
+
 // GET_T_GIVEN_EY, LiDryer.H:833-888: bounded Newton for T from e on NASA-7.
 // The mixture energy sum_n rho_n e_n(T) / W_n is one polynomial in T per
 // temperature range: its six coefficients are summed once (and again where an
 // iterate crosses 1000 K), so an iteration takes one Horner scheme with its
 // derivative (10 FMAs) instead of nine species' polynomials (about 190 FP64
-// operations of e and cv).  The same iterates up to rounding.  The step's
-// tests are integer compares of |dt|'s bits (FP64 compares run on the FP64
-// pipe); a NaN passes them as it passes the reference's.
+// operations of e and cv).  The same iterates up to rounding (some 1e-12 K).  The
+// reference drops a last step below 1e-7 K, so where that rounding decides - a step
+// within 1e-11 K of the tolerance, one cell in 1e5 or so - the loop is run again in
+// the reference's order and both end on the same iterate.  The step's tests are
+// integer compares of |dt|'s bits (FP64 compares run on the FP64 pipe); a NaN passes
+// them as it passes the reference's.
 __device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, double Ru) {
     const int maxiter = 200;
     const double ein = e, tmin = 250, tmax = 3500;
@@ -152,6 +171,7 @@ __device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, d
     double t1 = es * rcp_nr(As);
     if (t1 < tmin || t1 > tmax) t1 = tmin + (tmax - tmin) / (emax - emin) * (ein - emin);
     const long long mag = 0x7fffffffffffffffLL;
+    const double t0 = t1;
     int h = -1;
     double C[6];
     for (int i = 0; i < maxiter; ++i) {
@@ -178,7 +198,8 @@ __device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, d
         if (m > 0x4059000000000000LL) {  // |dt| > 100 (or NaN)
             if (dt > 100.0) dt = 100.0;
             else if (dt < -100.0) dt = -100.0;
-        } else if (m < 0x3E7AD7F29ABCAF48LL) {  // |dt| < 1e-7
+        } else if (m < 0x3E7AD8A286BBBB13LL) {  // |dt| < 1e-7 + 1e-11
+            if (m > 0x3E7AD742AEBDA37DLL) return newton_reference_order(ein, rhoi, Ru, t0);  // > 1e-7 - 1e-11
             break;
         }
         t1 += dt;
