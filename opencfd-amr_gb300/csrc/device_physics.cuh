@@ -7,6 +7,7 @@
 #pragma once
 
 #include "ocfd_internal.h"
+#include "weno_weights.cuh"
 
 namespace ocfd {
 
@@ -133,17 +134,6 @@ __device__ __forceinline__ double rcp_nr(double x) {
     return fma(r, e, r);
 }
 
-// a / b to within about one ulp for a normal, finite, non-zero b: the seed above
-// (relative error e) corrected by its cubic series, a r (1 + e + e^2), which is
-// good to e^3: four FP64 operations where rcp_nr and a product take five
-__device__ __forceinline__ double div_nr(double a, double b) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    const double e = __fma_rn(-b, r, 1.0);
-    const double q = __dmul_rn(a, r);
-    return __fma_rn(q, __fma_rn(e, e, e), q);
-}
-
 // WENO-Z of one split flux (Source/kernel/Reconstruction.H:83-138) in the fewest
 // FP64 operations (GB300 issues two FP64 instructions per cycle per SM).  The
 // stencil V1..V5 is ordered towards the face (f+: cells i-3..i+1; f-: cells
@@ -155,20 +145,20 @@ __device__ __forceinline__ double div_nr(double a, double b) {
 //     beta_2 = d2^2 + e2 (d2 + 4/3 e2), beta_3 = d3^2 + e3 (4/3 e3 - d3).
 //   - The weights alpha_k = c_k (1 + (tau / D_k)^2), D_k = eps + beta_k, c = (1, 6,
 //     3), are multiplied by the common positive factor (D_1 D_2 D_3)^2, which
-//     cancels in alpha_k / sum alpha: with q_k = D_k^2 and P = q_1 q_2 q_3, alpha_k
-//     becomes c_k A_k, A_k = P + tau^2 q_j q_l ({j, l} the other two).
+//     cancels in alpha_k / sum alpha: with q_k = D_k^2, alpha_k becomes c_k A_k,
+//     A_k = q_j q_l (q_k + tau^2) ({j, l} the other two), formed on the integer
+//     pipes (weno_weights.cuh).
 //   - The candidate polynomials are V3 + (3 d2 + 2 e1) / 6, V3 + (3 d2 + 2 e2) / 6
 //     and V3 + (3 d2 + 3 e2 - e3) / 6, so the face value is
 //     V3 + d2 / 2 + (2 A_1 e1 + 12 A_2 e2 + 3 A_3 (3 e2 - e3)) / (6 sum c_k A_k):
-//     three products and one division, and the rounding of the weights multiplies
-//     second differences only.
-// The same value up to rounding (parity tests: 1e-12 per right-hand side); the
-// products stay finite for |beta| < 2e50, i.e. flux differences below ~1e25.
-// Differences, and S = eps + d^2, belong to cells of the line and serve
-// neighbouring faces: 37 FP64 operations per face and side in runs of three faces
-// (42 for a face alone), against 49 (54) for indicators and candidates formed from
-// the values; a stage of the 3D blast on 128x128x64 cells took 4.00 ms that way and
-// 3.32 ms this way.
+//     three products, and the rounding of the weights multiplies second
+//     differences only.
+// The same value up to rounding (parity tests: 1e-12 per right-hand side), finite
+// for flux differences below ~1e150.  Differences, and S = eps + d^2, belong to
+// cells of the line and serve neighbouring faces: 18.5 FP64 operations per face
+// and side in runs of three faces (24 for a face alone).  With indicators and
+// candidates formed from the values and all of it in FP64 they were 49 (54), and a
+// stage of the 3D blast on 128x128x64 cells took 4.00 ms; this way 2.17 ms.
 // Every rounding is written out, so the value does not depend on the code around
 // the call.
 __device__ __forceinline__ double wenoz_s(double d) { return __fma_rn(d, d, 1e-6); }
@@ -177,15 +167,10 @@ __device__ __forceinline__ double wenoz_face_d(double V3, double d2, double d3, 
     const double D1 = __fma_rn(e1, __fma_rn(4.0 / 3.0, e1, d2), S2);
     const double D2 = __fma_rn(e2, __fma_rn(4.0 / 3.0, e2, d2), S2);
     const double D3 = __fma_rn(e3, __fma_rn(4.0 / 3.0, e3, -d3), S3);
-    const double tau = __dsub_rn(D1, D3);
-    const double q1 = __dmul_rn(D1, D1), q2 = __dmul_rn(D2, D2), q3 = __dmul_rn(D3, D3), t2 = __dmul_rn(tau, tau);
-    const double q12 = __dmul_rn(q1, q2), q13 = __dmul_rn(q1, q3), q23 = __dmul_rn(q2, q3);
-    const double Pq = __dmul_rn(q12, q3);
-    const double A1 = __fma_rn(t2, q23, Pq), A2 = __fma_rn(t2, q13, Pq), A3 = __fma_rn(t2, q12, Pq);
-    const double a2 = __dmul_rn(6.0, A2), a3 = __dmul_rn(1.5, A3);
-    const double num = __fma_rn(a3, __fma_rn(3.0, e2, -e3), __fma_rn(a2, e2, __dmul_rn(A1, e1)));
-    const double den = __fma_rn(2.0, a3, __dadd_rn(A1, a2));
-    return __fma_rn(div_nr(num, den), 1.0 / 3.0, __fma_rn(0.5, d2, V3));
+    double c1, c2, c3;
+    wz::weights(D1, D2, D3, fabs(__dsub_rn(D1, D3)), c1, c2, c3);
+    const double corr = __fma_rn(c3, __fma_rn(3.0, e2, -e3), __fma_rn(c2, e2, __dmul_rn(c1, e1)));
+    return __dadd_rn(__fma_rn(0.5, d2, V3), corr);
 }
 __device__ __forceinline__ double wenoz_1rcp(double V1, double V2, double V3, double V4, double V5) {
     const double d1 = __dsub_rn(V2, V1), d2 = __dsub_rn(V3, V2), d3 = __dsub_rn(V4, V3), d4 = __dsub_rn(V5, V4);
