@@ -396,7 +396,7 @@ ocfd_status level_autotune(ocfd_level* L, unsigned flags, int reps, cudaStream_t
     float best = 1e30f;
     int bt = L->tile, bs = L->sched;
     ocfd_status s = OCFD_OK;
-    for (int t = 0; t < kNumRegularTiles && s == OCFD_OK; ++t) {
+    for (int t = 0; t < kNumPublicTiles && s == OCFD_OK; ++t) {
         if (!regular_tile_fits(t, visc)) continue;
         if (kRegularTiles[t].staged && (!f32 || visc)) continue;  // the pencil kernel again
         L->tile = t;
@@ -684,22 +684,13 @@ ocfd_status level_alloc(ocfd_context* ctx, const ocfd_level_desc* desc, int nbuf
         L->zvirt_allowed = simple;
     }
     std::memcpy(L->bcinfo.params, desc->case_params, sizeof(L->bcinfo.params));
-    // RHS tile: the shape with the least padded work summed over the boxes
-    if (desc->tile >= 0 && desc->tile < kNumRegularTiles) {
+    if (desc->tile >= 0 && desc->tile < kNumPublicTiles) {
         L->tile = desc->tile;
     } else {
-        double best = 1e300;
-        for (int t = 0; t < kNumRegularTiles; ++t) {
-            if (!regular_tile_fits(t, true) || kRegularTiles[t].staged) continue;
-            const TileShape& ts = kRegularTiles[t];
-            double cost = 0;
-            for (const ocfd_box& B : L->boxes) {
-                const int n[3] = {B.hi[0] - B.lo[0] + 1, B.hi[1] - B.lo[1] + 1, B.hi[2] - B.lo[2] + 1};
-                long long tiles = (long long)((n[0] + ts.x - 1) / ts.x) * ((n[1] + ts.y - 1) / ts.y) * ((n[2] + ts.z - 1) / ts.z);
-                cost += tiles * ((double)ts.x * ts.y * ts.z * 3.0 + 6.0 * ((double)ts.y * ts.z + (double)ts.x * ts.z + (double)ts.x * ts.y));
-            }
-            if (cost < best * 0.999) { best = cost; L->tile = t; }
-        }
+        std::vector<int> n;
+        for (const ocfd_box& B : L->boxes)
+            for (int d = 0; d < 3; ++d) n.push_back(B.hi[d] - B.lo[d] + 1);
+        L->tile = pick_level_tile(reinterpret_cast<const int(*)[3]>(n.data()), (int)L->boxes.size(), ctx->num_sms);
     }
     if (s == OCFD_OK) {
         L->d_step = static_cast<StepState*>(dev_alloc(sizeof(StepState), pool));
@@ -839,7 +830,7 @@ ocfd_status ocfd_level_state(ocfd_level* L, int ibox, ocfd_array4* out) {
 size_t ocfd_level_state_elems(const ocfd_level* L) { return L ? (size_t)L->elems : 0; }
 
 ocfd_status ocfd_level_set_schedule(ocfd_level* L, int32_t tile, int32_t sched) {
-    if (!L || sched < 0 || sched >= NUM_SCHED || tile < -1 || tile >= kNumRegularTiles ||
+    if (!L || sched < 0 || sched >= NUM_SCHED || tile < -1 || tile >= kNumPublicTiles ||
         (tile >= 0 && !regular_tile_fits(tile, false)))
         return fail(OCFD_BAD_ARG, "ocfd_level_set_schedule");
     L->sched = sched;

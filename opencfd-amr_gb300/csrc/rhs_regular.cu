@@ -17,8 +17,9 @@ ocfd_status configure_rhs_regular() { return configure_all<double>(); }
 bool regular_tile_fits(int tile, bool visc) { return tile_fits<double>(tile, visc); }
 
 const TileShape kRegularTiles[] = {{8, 8, 8, 0},  {8, 8, 4, 0}, {16, 8, 4, 0}, {16, 16, 2, 0}, {32, 8, 2, 0},
-                                   {16, 8, 2, 0}, {8, 8, 8, 1}, {8, 8, 4, 1}, {16, 8, 4, 1}};
+                                   {16, 8, 2, 0}, {8, 8, 8, 1}, {8, 8, 4, 1}, {16, 8, 4, 1}, {8, 4, 4, 0}, {4, 4, 4, 0},  {4, 4, 2, 0}};
 const int kNumRegularTiles = sizeof(kRegularTiles) / sizeof(kRegularTiles[0]);
+const int kNumPublicTiles = 9;
 
 ocfd_status launch_rhs_regular(int tile, bool visc, const RegBoxArgs* d_boxes,
                                const int* d_tile_start, int nbox, const RegBoxArgs& single,
@@ -26,19 +27,48 @@ ocfd_status launch_rhs_regular(int tile, bool visc, const RegBoxArgs* d_boxes,
     return launch_any<double>(tile, visc, d_boxes, d_tile_start, nbox, single, ntiles, P, st, sched, queue);
 }
 
-// Default tile for a box: the shape with the least padded work.
-int pick_regular_tile(const int n[3], bool visc) {
+// Warp instructions a tile takes on the pipe that bounds its form (FP64: FP64
+// instructions; FP32: all), from its counts of work items per sweep: WENO-Z runs of
+// three faces x component (FP64) or faces x component (FP32), split cells of the
+// pencils, primitives (of the cross, or of each pencil and the ring with viscosity)
+// and viscous faces.  The weights are those of the kernels' instruction counts.
+static double tile_work(const TileShape& s, bool visc, bool f32) {
+    const int T[3] = {s.x, s.y, s.z};
+    auto warps = [](int items) { return (items + 31) / 32; };
+    const double weno = f32 ? 150 : 115, split = f32 ? 70 : 41, prim = f32 ? 60 : 40, vface = f32 ? 120 : 95;
+    double w = 0;
+    int cross = T[0] * T[1] * T[2];
+    for (int d = 0; d < 3; ++d) {
+        const int line = T[(d + 1) % 3] * T[(d + 2) % 3], faces = T[d] + 1, pencil = (T[d] + 6) * line;
+        w += weno * warps(5 * line * (f32 ? faces : (faces + 2) / 3)) + split * warps(pencil);
+        if (visc || f32) w += prim * warps(pencil);
+        if (visc) w += vface * warps(faces * line);
+        cross += 6 * line;
+    }
+    if (visc) w += prim * warps((T[0] + 2) * (T[1] + 2) * (T[2] + 2));
+    else if (!f32) w += prim * warps(cross);
+    return w;
+}
+
+// Tile for a set of boxes: the shape that ends first on `sms` SMs.  The pipe that
+// bounds a tile is shared by the CTAs of an SM, so a launch of n tiles takes
+// ceil(n / sms) tiles' work: large tiles have the least halo work per cell, small
+// ones spread a small box over more SMs and leave a shorter last wave.  Measured: a
+// viscous FP64 box of 20x12x8 cells as six 8^3 tiles 207 us, as 60 tiles of 4x4x2
+// (then bound by the latency of three warps) 47 us; one of 13x97x5 cells 275 us
+// (with FP64 weights) and 44 us.  FP32 boxes take the pencil tiles: TMA staging of
+// the same shape is slower (a box of 128x96x64 cells 183 us staged, 158 us not; two
+// CTAs per SM against three).
+static int pick_tile(const int (*n)[3], int nbox, bool visc, bool f32, int ntile_shapes, int sms) {
     int best = 1;
     double best_cost = 1e300;
-    for (int t = 0; t < kNumRegularTiles; ++t) {
+    for (int t = 0; t < ntile_shapes; ++t) {
         if (!regular_tile_fits(t, visc) || kRegularTiles[t].staged) continue;
         const TileShape& s = kRegularTiles[t];
-        long long tiles = (long long)((n[0] + s.x - 1) / s.x) * ((n[1] + s.y - 1) / s.y) *
-                          ((n[2] + s.z - 1) / s.z);
-        // padded cells plus pencil halo work per tile (6 cells per direction)
-        double per_tile = (double)s.x * s.y * s.z * 3.0 +
-                          6.0 * ((double)s.y * s.z + (double)s.x * s.z + (double)s.x * s.y);
-        double cost = tiles * per_tile;
+        long long tiles = 0;
+        for (int b = 0; b < nbox; ++b)
+            tiles += (long long)((n[b][0] + s.x - 1) / s.x) * ((n[b][1] + s.y - 1) / s.y) * ((n[b][2] + s.z - 1) / s.z);
+        const double cost = (double)((tiles + sms - 1) / sms) * tile_work(s, visc, f32);
         if (cost < best_cost * 0.999) {
             best_cost = cost;
             best = t;
@@ -46,6 +76,13 @@ int pick_regular_tile(const int n[3], bool visc) {
     }
     return best;
 }
+
+int pick_regular_tile(const int n[3], bool visc, bool f32, int sms) {
+    const int one[1][3] = {{n[0], n[1], n[2]}};
+    return pick_tile(one, 1, visc, f32, kNumRegularTiles, sms);
+}
+
+int pick_level_tile(const int (*n)[3], int nbox, int sms) { return pick_tile(n, nbox, true, false, kNumPublicTiles, sms); }
 
 void fill_regular_args(RegBoxArgs& a, const ocfd_array4* S, const ocfd_array4* dSdt,
                        const ocfd_array4* flux, const ocfd_box& bx, const double dxinv[3],
@@ -68,15 +105,6 @@ void fill_regular_args(RegBoxArgs& a, const ocfd_array4* S, const ocfd_array4* d
     a.dt_ptr = nullptr;
     a.cfl_min = nullptr;
     encode_regular_tmaps(a, S, tile);
-}
-
-int staged_regular_tile(int tile) {
-    const TileShape& s = kRegularTiles[tile];
-    for (int t = 0; t < kNumRegularTiles; ++t)
-        if (kRegularTiles[t].staged && kRegularTiles[t].x == s.x && kRegularTiles[t].y == s.y &&
-            kRegularTiles[t].z == s.z)
-            return t;
-    return tile;
 }
 
 static bool g_regular_tma = true;
@@ -158,7 +186,7 @@ extern "C" ocfd_status ocfd_rhs_regular_box_f64(ocfd_context* ctx, const ocfd_ar
     DevParm P = ctx->parm;
     P.grav = (flags & OCFD_GRAVITY) ? kGravity : 0.0;
     const int n[3] = {bx.hi[0] - bx.lo[0] + 1, bx.hi[1] - bx.lo[1] + 1, bx.hi[2] - bx.lo[2] + 1};
-    const int tile = pick_regular_tile(n, (flags & OCFD_VISC) != 0);
+    const int tile = pick_regular_tile(n, (flags & OCFD_VISC) != 0, false, ctx->num_sms);
     RegBoxArgs a{};
     fill_regular_args(a, S, dSdt, flux, bx, dxinv, tile);
     const int ntiles = a.ntile[0] * a.ntile[1] * a.ntile[2];

@@ -20,6 +20,7 @@ struct TileShape {
 };
 extern const TileShape kRegularTiles[];
 extern const int kNumRegularTiles;
+extern const int kNumPublicTiles;  // the shapes levels, the autotuner and the C ABI choose from
 
 // Everything one box needs; a device array of these drives the batched form.
 struct RegBoxArgs {
@@ -186,9 +187,9 @@ __device__ __forceinline__ void block_cfl_atomic(const CflSpeeds& c, const doubl
 // g of the gravity source, Source/Advance.cpp:332
 constexpr double kGravity = -9.8;
 
-int pick_regular_tile(const int n[3], bool visc);
-// the TMA-staged variant of tile's shape, or tile itself when it has none
-int staged_regular_tile(int tile);
+int pick_regular_tile(const int n[3], bool visc, bool f32, int sms);
+// one tile shape for the batched launches over a level's boxes (sizes n)
+int pick_level_tile(const int (*n)[3], int nbox, int sms);
 bool regular_tile_fits(int tile, bool visc);
 ocfd_status configure_rhs_regular();
 ocfd_status configure_rhs_regular_f32();

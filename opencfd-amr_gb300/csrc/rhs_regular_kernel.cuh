@@ -66,6 +66,15 @@ struct Pencil {
     static constexpr int SMEM = 10 * N + 5 * NF;                       // elements
 };
 
+// threads of a tile's CTA: one per cell, and in small tiles enough for the WENO-Z
+// work items of a sweep (5 components x lines x runs of three faces)
+template <int TX, int TY, int TZ>
+__host__ __device__ constexpr int tile_threads() {
+    constexpr int ix = 5 * TY * TZ * ((TX + 3) / 3), iy = 5 * TX * TZ * ((TY + 3) / 3), iz = 5 * TX * TY * ((TZ + 3) / 3);
+    constexpr int items = ix > iy ? (ix > iz ? ix : iz) : (iy > iz ? iy : iz), cells = TX * TY * TZ;
+    return cells >= 256 ? cells : ((items > cells ? items : cells) + 31) / 32 * 32;
+}
+
 template <int TX, int TY, int TZ>
 struct Ring {
     static constexpr int RX = TX + 2, RY = TY + 2, RZ = TZ + 2;
@@ -309,7 +318,7 @@ template <int TX, int TY, int TZ>
 __device__ __forceinline__ void cross_prims(const RegBoxArgs& B, const DevParm& P, int i0, int j0, int k0,
                                             const double* stage, bool staged, float* Q) {
     using C = Cross<TX, TY, TZ>;
-    constexpr int NT = TX * TY * TZ;
+    constexpr int NT = tile_threads<TX, TY, TZ>();
     for (int idx = threadIdx.x; idx < C::NQ; idx += NT) {
         int x, y, z, so, sc;
         bool zhalo = false;
@@ -372,7 +381,7 @@ template <int TX, int TY, int TZ>
 __device__ __forceinline__ void cross_prims_plain(const RegBoxArgs& B, const DevParm& P, int i0, int j0, int k0,
                                                   double* Q) {
     using C = Cross<TX, TY, TZ>;
-    constexpr int NT = TX * TY * TZ;
+    constexpr int NT = tile_threads<TX, TY, TZ>();
     for (int idx = threadIdx.x; idx < C::NQ; idx += NT) {
         int x, y, z;
         if (idx < C::NC) {
@@ -416,8 +425,12 @@ template <class FT, int D, int TX, int TY, int TZ, bool VISC, bool CROSS = false
 __device__ __forceinline__ void sweep(const RegBoxArgs& B, const DevParm& P, int i0, int j0, int k0,
                                       FT* F, FT* FF, const FT* ring, FT* acc, const FT* Q = nullptr) {
     using PC = Pencil<D, TX, TY, TZ>;
-    constexpr int NT = TX * TY * TZ;
+    constexpr int NT = tile_threads<TX, TY, TZ>();
     const int tid = threadIdx.x;
+    // an FP64 tile that overhangs the box: its faces outside are not formed (nothing
+    // reads them; a box of 61x45x37 cells is a fifth padding in 8^3 tiles).  The FP32
+    // form, bound by instruction issue, lost 1 % on full tiles to the test.
+    const bool over = std::is_same<FT, double>::value && (i0 + TX - 1 > B.hi[0] || j0 + TY - 1 > B.hi[1] || k0 + TZ - 1 > B.hi[2]);
     // ---- 1. primitives and Steger-Warming split over the pencil (primitives
     // from Q when the cross was staged)
     if constexpr (CROSS) {
@@ -489,6 +502,7 @@ __device__ __forceinline__ void sweep(const RegBoxArgs& B, const DevParm& P, int
             } else {
                 fx = line % PC::FX; fy = line / PC::FX; fz = f0;
             }
+            if (over && (i0 + fx > B.hi[0] + (D == 0) || j0 + fy > B.hi[1] + (D == 1) || k0 + fz > B.hi[2] + (D == 2))) continue;
             const int f = fx + fy * PC::FX + fz * PC::FX * PC::FY;
             const int base = fx + fy * PC::PX + fz * PC::PX * PC::PY;
             // f+ then f- (one side's registers at a time); the face flux is
@@ -528,13 +542,14 @@ __device__ __forceinline__ void sweep(const RegBoxArgs& B, const DevParm& P, int
         const FT dxinvT[3] = {dxinv_of<FT>(B, 0), dxinv_of<FT>(B, 1), dxinv_of<FT>(B, 2)};
         for (int f = tid; f < PC::NF; f += NT) {
             const int fx = f % PC::FX, fy = (f / PC::FX) % PC::FY, fz = f / (PC::FX * PC::FY);
+            if (over && (i0 + fx > B.hi[0] + (D == 0) || j0 + fy > B.hi[1] + (D == 1) || k0 + fz > B.hi[2] + (D == 2))) continue;
             // ring coordinates of the cell on the high side of the face
             visc_face<FT, D, TX, TY, TZ>(P, ring, fx + 1, fy + 1, fz + 1, dxinvT, FF + f, PC::NF);
         }
         __syncthreads();
     }
     // ---- 4. divergence contribution and optional face-flux output
-    {
+    if (NT == TX * TY * TZ || tid < TX * TY * TZ) {
         const int ti = tid % TX, tj = (tid / TX) % TY, tk = tid / (TX * TY);
         const int f = ti + tj * PC::FX + tk * PC::FX * PC::FY;
         const FT dxi = dxinv_of<FT>(B, D);
@@ -596,7 +611,7 @@ __device__ __forceinline__ void rhs_tile(const RegBoxArgs* __restrict__ boxes, c
                                          int nbox, const RegBoxArgs& single, const DevParm& P, int t,
                                          unsigned char* sbase, uint64_t* bar, uint32_t& phase, bool& abort,
                                          double& local_dt) {
-    constexpr int NT = TX * TY * TZ;
+    constexpr int NT = tile_threads<TX, TY, TZ>();
     // locate the box of this tile: a single box, or a prefix table over a box list
     int b = 0;
     if (boxes) {
@@ -697,7 +712,7 @@ __device__ __forceinline__ void rhs_tile(const RegBoxArgs* __restrict__ boxes, c
 
     const int ti = threadIdx.x % TX, tj = (threadIdx.x / TX) % TY, tk = threadIdx.x / (TX * TY);
     const int ci = i0 + ti, cj = j0 + tj, ck = k0 + tk;
-    const bool valid = ci <= B.hi[0] && cj <= B.hi[1] && ck <= B.hi[2];
+    const bool valid = (NT == TX * TY * TZ || (int)threadIdx.x < TX * TY * TZ) && ci <= B.hi[0] && cj <= B.hi[1] && ck <= B.hi[2];
     if (valid) {
         double L[5];
 #pragma unroll
@@ -747,14 +762,14 @@ template <class FT, int TX, int TY, int TZ, bool VISC, bool XS>
 __host__ __device__ constexpr int regular_min_blocks() {
     if (std::is_same<FT, double>::value) return 1;  // the FP64 WENO-Z runs hold a sliding window
     const int b = (int)((228u * 1024u) / (regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>() + 1024u));
-    const int t = 2048 / (TX * TY * TZ);
+    const int t = 2048 / tile_threads<TX, TY, TZ>();
     int m = b < t ? b : t;
     m = m < 3 ? m : 3;
     return m < 1 ? 1 : m;
 }
 
 template <class FT, int TX, int TY, int TZ, bool VISC, bool XS>
-__global__ void __launch_bounds__(TX* TY* TZ, (regular_min_blocks<FT, TX, TY, TZ, VISC, XS>()))
+__global__ void __launch_bounds__((tile_threads<TX, TY, TZ>()), (regular_min_blocks<FT, TX, TY, TZ, VISC, XS>()))
     k_rhs_regular(const RegBoxArgs* __restrict__ boxes, const int* __restrict__ tile_start,
                   int nbox, const __grid_constant__ RegBoxArgs single, DevParm P, int ntiles, int sched,
                   unsigned* queue) {
@@ -810,7 +825,7 @@ template <class FT, int TX, int TY, int TZ, bool VISC, bool XS>
 static ocfd_status launch_t(const RegBoxArgs* d_boxes, const int* d_tile_start, int nbox,
                             const RegBoxArgs& single, int ntiles, const DevParm& P,
                             cudaStream_t st, int sched, unsigned* queue) {
-    constexpr int NT = TX * TY * TZ;
+    constexpr int NT = tile_threads<TX, TY, TZ>();
     constexpr size_t smem = regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>();
     auto kern = k_rhs_regular<FT, TX, TY, TZ, VISC, XS>;
     if (smem > kMaxSmem) return fail(OCFD_BAD_ARG, "regular RHS tile does not fit shared memory in this mode");
@@ -844,10 +859,13 @@ static bool configure_one() {
 // Every compiled tile: index (position in kRegularTiles), shape, and whether it
 // is the TMA-staged variant (XS) of its shape.  A staged index runs the staged
 // kernel only in the inviscid FP32-flux form; in every other mode it runs the
-// pencil kernel of its shape (the same instantiation as the plain index).
+// pencil kernel of its shape (the same instantiation as the plain index).  The
+// shapes from kNumPublicTiles on serve the per-box calls on boxes too small to give
+// every SM a larger tile.
 #define OCFD_REGULAR_TILES(X)                                                                              \
     X(0, 8, 8, 8, false) X(1, 8, 8, 4, false) X(2, 16, 8, 4, false) X(3, 16, 16, 2, false) X(4, 32, 8, 2, false) \
-        X(5, 16, 8, 2, false) X(6, 8, 8, 8, true) X(7, 8, 8, 4, true) X(8, 16, 8, 4, true)
+        X(5, 16, 8, 2, false) X(6, 8, 8, 8, true) X(7, 8, 8, 4, true) X(8, 16, 8, 4, true)                          \
+    X(9, 8, 4, 4, false) X(10, 4, 4, 4, false) X(11, 4, 4, 2, false)
 
 template <class FT>
 struct StagedIn {  // the staged variants exist in the FP32-flux form only
