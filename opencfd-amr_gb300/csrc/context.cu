@@ -12,6 +12,7 @@
 
 namespace ocfd {
 
+ocfd_status configure_chem();
 
 static thread_local std::string g_last_error;
 
@@ -164,6 +165,7 @@ ocfd_status ocfd_context_create(const ocfd_parm* parm, int device, ocfd_context*
     if (s == OCFD_OK) s = configure_rhs_regular();
     if (s == OCFD_OK) s = configure_rhs_regular_f32();
     if (s == OCFD_OK) s = configure_eb_tile();
+    if (s == OCFD_OK) s = configure_chem();
     if (s == OCFD_OK) s = eb_static_scratch_resolve(ctx);
     if (s != OCFD_OK) {
         cudaFree(ctx->d_error);

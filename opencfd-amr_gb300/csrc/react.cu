@@ -319,7 +319,7 @@ static ocfd_status record_react_step(ocfd_react* R, unsigned flags, cudaStream_t
             const ChemBoxArgs& A = R->args[in][b];
             if (!R->cls.empty() && R->cls[b] == OCFD_BOX_COVERED) continue;  // dSdt = 0 (Advance.cpp:213-214)
             s = A.eb ? launch_chem_eb_rhs(A, R->ctx->parm, sms, st) : launch_chem_rhs(A, R->ctx->parm, sms, st);
-            launches += A.visc ? 6 : 5;
+            launches += (A.eb ? 5 : 3) + (A.visc ? 1 : 0);
         }
         if (s != OCFD_OK) break;
         k_react_combine<<<grid_for(L->ncells, 256, sms), 256, 0, st>>>(
