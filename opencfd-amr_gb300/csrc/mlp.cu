@@ -128,49 +128,38 @@ __global__ void k_mlp_pack(const float* __restrict__ X, uint16_t* Xb, long long 
     }
 }
 
-// loss = mean over rows and the 10 outputs of (Y - T)^2; dY = dloss / dY into
-// dZ4 [M x 16] (zero on the padding); per-block partial sums of the loss
-__global__ void k_mlp_out_grad(const float* __restrict__ Y, const float* __restrict__ T, float* dZ4, long long M,
-                               float* lossp) {
-    __shared__ float red[256];
-    float acc = 0.0f;
-    const float scale = 2.0f / (float)(M * MLP_OUT);
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < M * 16;
-         e += (long long)gridDim.x * blockDim.x) {
-        const long long m = e >> 4;
-        const int j = (int)(e & 15);
-        float g = 0.0f;
-        if (j < MLP_OUT) {
-            const float d = Y[e] - T[m * MLP_OUT + j];
-            acc += d * d;
-            g = scale * d;
-        }
-        dZ4[e] = g;
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) lossp[blockIdx.x] = red[0];
-}
+// Backward pass of the activations, one 128-row tile through all layers (the tile
+// routine's mirror image): the output gradient dZ_4 = dloss / dY of loss = mean over
+// rows and the 10 outputs of (Y - T)^2, then for l = 4..1 the product dZ_l W_l on the
+// tensor cores (A = dZ_l 128 x N_l, B(j, n) = W_l[n][j]) times gelu'(Z_{l-1}) in the
+// epilogue, which stores dZ_{l-1} in FP32 for the weight gradients and, as BF16, as
+// the next product's A operand.  The transposed weights of all four layers (100 KB)
+// are staged once per CTA; four warpgroups share a tile's epilogue by columns, which
+// bounds it (erf, exp).  A training step's batch of 8192 rows: four launches of one
+// warpgroup per tile, each staging its weights element by element, 164 us, this one
+// 36 us.
+// lossp[block] = the block's share of the sum of squares.
+constexpr int SD_W = 0;                                 // W_1^T .. W_3^T, then W_4^T (128 x 16)
+constexpr int SD_A = 3 * 128 * 128 * 2 + 128 * 16 * 2;  // dZ_l, BF16
+constexpr int SD_BAR = SD_A + 128 * 128 * 2, SD_RED = SD_BAR + 16, SD_TOT = SD_RED + 4 * 4;
+__host__ __device__ constexpr int sd_w(int l) { return SD_W + (l - 1) * 128 * 128 * 2; }
 
-// dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1}) for layer l = 1..4, 128-row tiles:
-// A = dZ_l (128 x N_l, BF16), B(j, n) = W_l[n][j] (K_l x N_l), D = 128 x 128
-constexpr int SD_A = 0, SD_B = 128 * 128 * 2, SD_BAR = 2 * 128 * 128 * 2, SD_TOT = SD_BAR + 16;
-
-__global__ void __launch_bounds__(128) k_mlp_bwd_data(MlpNet net, int l, const float* __restrict__ dZl,
-                                                      const float* __restrict__ Zprev, float* dZprev, int ntile,
-                                                      unsigned* err) {
+__global__ void __launch_bounds__(MLP_THREADS) k_mlp_bwd(const uint16_t* __restrict__ Wt, const float* __restrict__ Y,
+                                                         const float* __restrict__ T, const float* __restrict__ Z,
+                                                         float* dZ4, float* dZ, float* lossp, int ntile, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + SD_BAR);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + SD_BAR + 8);
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int N = LN(l), K = LK(l);  // this layer: N outputs, K inputs (= 128)
-    for (int e = tid; e < N * K; e += 128) {
-        const int n = e / K, j = e % K;
-        *reinterpret_cast<uint16_t*>(sm + SD_B + kmajor_offset(j, n, K)) = net.W[WOFF(l) + e];
+    float* red = reinterpret_cast<float*>(sm + SD_RED);
+    const int tid = threadIdx.x, warp = tid >> 5, lrow = tid & 127, cg = tid >> 7;
+    for (int l = 1; l < 5; ++l) {
+        const int N = LN(l);  // K extent of the product (this layer's outputs)
+        const uint16_t* src = Wt + WOFF(l);
+        for (int q = tid; q < 128 * N / 8; q += MLP_THREADS) {
+            const int j = q / (N / 8), n = (q % (N / 8)) * 8;
+            *reinterpret_cast<uint4*>(sm + sd_w(l) + kmajor_offset(j, n, 128)) =
+                __ldg(reinterpret_cast<const uint4*>(src + (long long)j * N + n));
+        }
     }
     if (tid == 0) mbar_init(bar, 1);
     if (warp == 0) {
@@ -181,78 +170,172 @@ __global__ void __launch_bounds__(128) k_mlp_bwd_data(MlpNet net, int l, const f
     __syncthreads();
     fence_after_sync();
     const uint32_t tbase = *tslot;
-    const uint32_t trow = tbase + ((uint32_t)(warp * 32) << 16);
+    const uint32_t trow = tbase + ((uint32_t)((warp & 3) * 32) << 16);
+    const long long M = (long long)ntile * 128;
+    const float scale = 2.0f / (float)(M * MLP_OUT);
     uint32_t phase = 0;
     bool ok = true;
+    float acc = 0.0f;
     for (int t = blockIdx.x; t < ntile && ok; t += gridDim.x) {
-        const long long row = (long long)t * 128 + tid;
-        for (int n = 0; n < N; ++n)
-            *reinterpret_cast<uint16_t*>(sm + SD_A + kmajor_offset(tid, n, 128)) = bf16_bits(dZl[row * N + n]);
-        fence_async_smem();
-        fence_before_sync();
-        __syncthreads();
-        fence_after_sync();
-        if (tid == 0) {
-            const uint32_t idesc = idesc_bf16_f32(128, K);
-            for (int ks = 0; ks < N / 16; ++ks)
-                mma_bf16(tbase, smem_desc(smem_u32(sm + SD_A + ks * 128 * 32)),
-                         smem_desc(smem_u32(sm + SD_B + ks * K * 32)), idesc, ks > 0 ? 1u : 0u);
-            mma_commit(bar);
-        }
-        ok = mbar_wait(bar, phase);
-        phase ^= 1u;
-        fence_after_sync();
-        if (!ok) break;
-        for (int c0 = 0; c0 < 128; c0 += 32) {
-            float v[32];
-            tmem_ld32(trow + (uint32_t)c0, v);
+        const long long row = (long long)t * 128 + lrow;
+        if (tid < 128) {
+            float g[16];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const long long q = row * 128 + c0 + i;
-                dZprev[q] = v[i] * gelu_grad(Zprev[q]);
+            for (int q = 0; q < 4; ++q) {
+                const float4 y = *reinterpret_cast<const float4*>(Y + row * 16 + 4 * q);
+                g[4 * q] = y.x;
+                g[4 * q + 1] = y.y;
+                g[4 * q + 2] = y.z;
+                g[4 * q + 3] = y.w;
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (j < MLP_OUT) {
+                    const float d = g[j] - T[row * MLP_OUT + j];
+                    acc += d * d;
+                    g[j] = scale * d;
+                } else {
+                    g[j] = 0.0f;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<float4*>(dZ4 + row * 16 + 4 * q) =
+                    make_float4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
+#pragma unroll
+            for (int q = 0; q < 16; q += 8)
+                *reinterpret_cast<uint4*>(sm + SD_A + kmajor_offset(lrow, q, 128)) =
+                    make_uint4(bf16x2_bits(g[q], g[q + 1]), bf16x2_bits(g[q + 2], g[q + 3]),
+                               bf16x2_bits(g[q + 4], g[q + 5]), bf16x2_bits(g[q + 6], g[q + 7]));
+        }
+        for (int l = 4; l >= 1; --l) {
+            fence_async_smem();
+            fence_before_sync();
+            __syncthreads();
+            fence_after_sync();
+            if (tid == 0) {
+                const uint32_t idesc = idesc_bf16_f32(128, 128);
+                for (int ks = 0; ks < LN(l) / 16; ++ks)
+                    mma_bf16(tbase, smem_desc(smem_u32(sm + SD_A + ks * 128 * 32)),
+                             smem_desc(smem_u32(sm + sd_w(l) + ks * 128 * 32)), idesc, ks > 0 ? 1u : 0u);
+                mma_commit(bar);
+            }
+            ok = mbar_wait(bar, phase);
+            phase ^= 1u;
+            fence_after_sync();
+            if (!ok) break;
+            const long long q0 = (long long)(l - 1) * M * 128 + row * 128 + cg * 32;
+            float v[32];
+            tmem_ld32(trow + (uint32_t)(cg * 32), v);
+#pragma unroll
+            for (int c = 0; c < 32; c += 8) {
+                const float4 za = *reinterpret_cast<const float4*>(Z + q0 + c);
+                const float4 zb = *reinterpret_cast<const float4*>(Z + q0 + c + 4);
+                const float z[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[c + i] *= gelu_grad(z[i]);
+                *reinterpret_cast<float4*>(dZ + q0 + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                *reinterpret_cast<float4*>(dZ + q0 + c + 4) = make_float4(v[c + 4], v[c + 5], v[c + 6], v[c + 7]);
+                if (l > 1)
+                    *reinterpret_cast<uint4*>(sm + SD_A + kmajor_offset(lrow, cg * 32 + c, 128)) =
+                        make_uint4(bf16x2_bits(v[c], v[c + 1]), bf16x2_bits(v[c + 2], v[c + 3]),
+                                   bf16x2_bits(v[c + 4], v[c + 5]), bf16x2_bits(v[c + 6], v[c + 7]));
             }
         }
         fence_before_sync();
         __syncthreads();
     }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (tid < 128 && (tid & 31) == 0) red[warp] = acc;
     if (!ok && tid == 0) atomicOr(err, 1u);
     fence_before_sync();
     __syncthreads();
+    if (tid == 0) lossp[blockIdx.x] = red[0] + red[1] + red[2] + red[3];
     if (warp == 0) tmem_dealloc(tbase, 128);
 }
 
-// Weight and bias gradients of layer l over one chunk of 256 rows (block c):
+// Weight and bias gradients of layer blockIdx.y over one chunk of 128 rows (block x):
 // dW_l[n][k] = sum_m dZ_l[m][n] A_l[m][k], db_l[n] = sum_m dZ_l[m][n], as
 // partials partW[c][.], partb[c][.].  The tensor-core M dimension (128 rows)
 // is n for l < 4 and k for l = 4 (whose N_l = 16); the MMA K dimension is the
-// chunk's rows.
-constexpr int CHUNK = 256;
-constexpr int SW_A = 0, SW_B = 128 * CHUNK * 2, SW_BAR = 2 * 128 * CHUNK * 2, SW_TOT = SW_BAR + 16;
+// chunk's rows, so both operands are the transposes of row-major arrays: a thread
+// gathers two columns of eight rows (coalesced across the warp's columns) into two
+// 16-byte core-matrix rows.  64 KB of operands, three CTAs per SM; all five layers
+// in one launch (8192 rows: 320 CTAs, 20 us; five launches of 32 CTAs gathering
+// element by element took 231 us).
+constexpr int CHUNK = 128;       // rows per weight-gradient block
+constexpr int BATCH_ROWS = 256;  // training batches are multiples of this
+constexpr int WG_THREADS = 256;
+constexpr int SW_A = 0, SW_B = 128 * CHUNK * 2, SW_RED = 2 * 128 * CHUNK * 2, SW_BAR = SW_RED + 4 * 128 * 4,
+              SW_TOT = SW_BAR + 16;
 
-__global__ void __launch_bounds__(128) k_mlp_bwd_weight(int l, const float* __restrict__ dZl,
-                                                        const uint16_t* __restrict__ Al, int lda, float* partW,
-                                                        float* partb, unsigned* err) {
+// columns of src [rows m0.. x ld] as a K-major operand of `ncol` rows; FP32 sources
+// also leave the sums of their columns over the chunk in red[4][ncol]
+__device__ __forceinline__ void stage_columns(unsigned char* dst, const float* __restrict__ src, int ncol, float* red) {
+    const int np = ncol / 2;
+    for (int it = threadIdx.x; it < np * 4; it += WG_THREADS) {
+        const int p = it % np, g = it / np;  // column pair, quarter of the rows
+        float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+        for (int o = 0; o < CHUNK / 32; ++o) {
+            const int mm = (g * (CHUNK / 32) + o) * 8;
+            float2 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const float2*>(src + (long long)(mm + i) * ncol + 2 * p);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                s0 += v[i].x;
+                s1 += v[i].y;
+            }
+            *reinterpret_cast<uint4*>(dst + kmajor_offset(2 * p, mm, ncol)) =
+                make_uint4(bf16x2_bits(v[0].x, v[1].x), bf16x2_bits(v[2].x, v[3].x), bf16x2_bits(v[4].x, v[5].x),
+                           bf16x2_bits(v[6].x, v[7].x));
+            *reinterpret_cast<uint4*>(dst + kmajor_offset(2 * p + 1, mm, ncol)) =
+                make_uint4(bf16x2_bits(v[0].y, v[1].y), bf16x2_bits(v[2].y, v[3].y), bf16x2_bits(v[4].y, v[5].y),
+                           bf16x2_bits(v[6].y, v[7].y));
+        }
+        red[g * ncol + 2 * p] = s0;
+        red[g * ncol + 2 * p + 1] = s1;
+    }
+}
+__device__ __forceinline__ void stage_columns(unsigned char* dst, const uint16_t* __restrict__ src, int ncol) {
+    const int np = ncol / 2;
+    for (int it = threadIdx.x; it < np * (CHUNK / 8); it += WG_THREADS) {
+        const int p = it % np, mm = it / np * 8;
+        uint32_t v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const uint32_t*>(src + (long long)(mm + i) * ncol + 2 * p);
+        uint4 lo, hi;
+        lo.x = __byte_perm(v[0], v[1], 0x5410);
+        lo.y = __byte_perm(v[2], v[3], 0x5410);
+        lo.z = __byte_perm(v[4], v[5], 0x5410);
+        lo.w = __byte_perm(v[6], v[7], 0x5410);
+        hi.x = __byte_perm(v[0], v[1], 0x7632);
+        hi.y = __byte_perm(v[2], v[3], 0x7632);
+        hi.z = __byte_perm(v[4], v[5], 0x7632);
+        hi.w = __byte_perm(v[6], v[7], 0x7632);
+        *reinterpret_cast<uint4*>(dst + kmajor_offset(2 * p, mm, ncol)) = lo;
+        *reinterpret_cast<uint4*>(dst + kmajor_offset(2 * p + 1, mm, ncol)) = hi;
+    }
+}
+
+__global__ void __launch_bounds__(WG_THREADS) k_mlp_bwd_weight(const float* __restrict__ dZ4, const float* __restrict__ dZ,
+                                                               const uint16_t* __restrict__ Xb,
+                                                               const uint16_t* __restrict__ H, long long M, float* partW,
+                                                               float* partb, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + SW_BAR);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + SW_BAR + 8);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    float* red = reinterpret_cast<float*>(sm + SW_RED);
+    const int tid = threadIdx.x, warp = tid >> 5, l = blockIdx.y;
     const int N = LN(l), K = LK(l);
     const long long m0 = (long long)blockIdx.x * CHUNK;
     const bool swap = (l == 4);
     const int ncol = swap ? N : K;  // columns of D
-    // A: 128 rows (n, or k when swapped) x CHUNK; B: ncol rows x CHUNK
-    for (int e = tid; e < 128 * CHUNK; e += 128) {
-        const int r = e / CHUNK, mm = e % CHUNK;
-        const long long m = m0 + mm;
-        const uint16_t v = swap ? Al[m * lda + r] : bf16_bits(dZl[m * N + r]);
-        *reinterpret_cast<uint16_t*>(sm + SW_A + kmajor_offset(r, mm, 128)) = v;
-    }
-    for (int e = tid; e < ncol * CHUNK; e += 128) {
-        const int r = e / CHUNK, mm = e % CHUNK;
-        const long long m = m0 + mm;
-        const uint16_t v = swap ? bf16_bits(dZl[m * N + r]) : Al[m * lda + r];
-        *reinterpret_cast<uint16_t*>(sm + SW_B + kmajor_offset(r, mm, ncol)) = v;
-    }
+    const float* dz = (l == 4 ? dZ4 : dZ + (long long)l * M * 128) + m0 * N;
+    const uint16_t* in = (l == 0 ? Xb : H + (long long)(l - 1) * M * 128) + m0 * K;
+    stage_columns(sm + (swap ? SW_B : SW_A), dz, N, red);
+    stage_columns(sm + (swap ? SW_A : SW_B), in, K);
     if (tid == 0) mbar_init(bar, 1);
     if (warp == 0) {
         tmem_alloc(tslot, 128);
@@ -270,26 +353,27 @@ __global__ void __launch_bounds__(128) k_mlp_bwd_weight(int l, const float* __re
                      smem_desc(smem_u32(sm + SW_B + ks * ncol * 32)), idesc, ks > 0 ? 1u : 0u);
         mma_commit(bar);
     }
-    // bias partial while the tensor core works: rows of the chunk in order
-    if (tid < N) {
-        float acc = 0.0f;
-        for (int mm = 0; mm < CHUNK; ++mm) acc += dZl[(m0 + mm) * N + tid];
-        partb[(long long)blockIdx.x * BTOT + BOFF(l) + tid] = acc;
-    }
+    if (tid < N)
+        partb[(long long)blockIdx.x * BTOT + BOFF(l) + tid] =
+            (red[tid] + red[N + tid]) + (red[2 * N + tid] + red[3 * N + tid]);
     const bool ok = mbar_wait(bar, 0);
     fence_after_sync();
     if (!ok) {
         if (tid == 0) atomicOr(err, 1u);
     } else {
         float* pw = partW + (long long)blockIdx.x * WTOT + WOFF(l);
-        for (int c0 = 0; c0 < ncol; c0 += 16) {
+        const int r = (warp & 3) * 32 + (tid & 31);
+        for (int c0 = (warp >> 2) * 16; c0 < ncol; c0 += 32) {
             float v[16];
-            tmem_ld16(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+            tmem_ld16(tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
+            // row r, columns c0.. of D
+            if (swap) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                // row tid, column c0 + i of D
-                if (swap) pw[(c0 + i) * K + tid] = v[i];   // D[k][n] -> W[n][k]
-                else pw[tid * K + c0 + i] = v[i];          // D[n][k]
+                for (int i = 0; i < 16; ++i) pw[(c0 + i) * K + r] = v[i];  // D[k][n] -> W[n][k]
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i += 4)  // D[n][k]
+                    *reinterpret_cast<float4*>(pw + r * K + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
             }
         }
     }
@@ -298,10 +382,17 @@ __global__ void __launch_bounds__(128) k_mlp_bwd_weight(int l, const float* __re
     if (warp == 0) tmem_dealloc(tbase, 128);
 }
 
+// element of W_1^T .. W_4^T (each N_l contiguous per input) of weight element q
+__device__ __forceinline__ int transposed_index(int q) {
+    const int l = q < WOFF(2) ? 1 : (q < WOFF(3) ? 2 : (q < WOFF(4) ? 3 : 4));
+    const int r = q - WOFF(l), N = LN(l);
+    return WOFF(l) + (r % 128) * N + r / 128;
+}
+
 // gradients = sum of the chunk partials in chunk order; Adam step on the FP32
 // master parameters (bias-corrected, Kingma & Ba 2015); BF16 copy of the weights
 __global__ void k_mlp_reduce_adam(const float* __restrict__ partW, const float* __restrict__ partb, int nchunk,
-                                  float* W32, float* b32, float* mW, float* vW, float* mb, float* vb, uint16_t* Wb,
+                                  float* W32, float* b32, float* mW, float* vW, float* mb, float* vb, uint16_t* Wb, uint16_t* Wt,
                                   float* gW, float* gb, float lr, float c1, float c2, int update) {
     const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < WTOT + BTOT; i += gridDim.x * blockDim.x) {
@@ -310,6 +401,7 @@ __global__ void k_mlp_reduce_adam(const float* __restrict__ partW, const float* 
         const float* part = isw ? partW : partb;
         const int stride = isw ? WTOT : BTOT;
         float g = 0.0f;
+#pragma unroll 8
         for (int c = 0; c < nchunk; ++c) g += part[(long long)c * stride + q];
         if (gW && isw) gW[q] = g;
         if (gb && !isw) gb[q] = g;
@@ -320,13 +412,18 @@ __global__ void k_mlp_reduce_adam(const float* __restrict__ partW, const float* 
         *m = beta1 * *m + (1.0f - beta1) * g;
         *v = beta2 * *v + (1.0f - beta2) * g * g;
         *p -= lr * (*m * c1) / (sqrtf(*v * c2) + eps);
-        if (isw) Wb[q] = bf16_bits(*p);
+        if (isw) {
+            Wb[q] = bf16_bits(*p);
+            if (q >= WOFF(1)) Wt[transposed_index(q)] = Wb[q];
+        }
     }
 }
 
-__global__ void k_mlp_to_bf16(const float* W32, uint16_t* Wb) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < WTOT; i += gridDim.x * blockDim.x)
+__global__ void k_mlp_to_bf16(const float* W32, uint16_t* Wb, uint16_t* Wt) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < WTOT; i += gridDim.x * blockDim.x) {
         Wb[i] = bf16_bits(W32[i]);
+        if (i >= WOFF(1)) Wt[transposed_index(i)] = Wb[i];
+    }
 }
 
 }  // namespace ocfd
@@ -337,6 +434,7 @@ struct ocfd_mlp {
     int max_batch = 0;
     float *W32 = nullptr, *b32 = nullptr, *mW = nullptr, *vW = nullptr, *mb = nullptr, *vb = nullptr;
     uint16_t* Wb = nullptr;
+    uint16_t* Wt = nullptr;  // W_1 .. W_4 transposed, at the offsets of Wb
     float norm[2 * ocfd::MLP_IN + 3 * ocfd::MLP_OUT] = {};
     long long steps = 0;
     // training scratch (max_batch rows)
@@ -345,8 +443,7 @@ struct ocfd_mlp {
     float* Z = nullptr;      // 4 x M x 128
     uint16_t* H = nullptr;   // 4 x M x 128
     float* dZ4 = nullptr;    // M x 16
-    float* dZa = nullptr;    // M x 128
-    float* dZb = nullptr;    // M x 128
+    float* dZ = nullptr;     // 4 x M x 128
     float* partW = nullptr;  // nchunk x WTOT
     float* partb = nullptr;  // nchunk x BTOT
     float* lossp = nullptr;
@@ -379,7 +476,7 @@ static ocfd_status mlp_configure() {
     if (done) return OCFD_OK;
     if (cudaFuncSetAttribute(k_mlp_forward<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_tot(1)) != cudaSuccess ||
         cudaFuncSetAttribute(k_mlp_forward<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, s_tot(2)) != cudaSuccess ||
-        cudaFuncSetAttribute(k_mlp_bwd_data, cudaFuncAttributeMaxDynamicSharedMemorySize, SD_TOT) != cudaSuccess ||
+        cudaFuncSetAttribute(k_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, SD_TOT) != cudaSuccess ||
         cudaFuncSetAttribute(k_mlp_bwd_weight, cudaFuncAttributeMaxDynamicSharedMemorySize, SW_TOT) != cudaSuccess)
         return check_launch("MLP kernel attributes");
     done = true;
@@ -399,28 +496,13 @@ static ocfd_status mlp_forward(ocfd_mlp* n, const float* X, long long M, cudaStr
     return check_launch("MLP forward");
 }
 
-static ocfd_status mlp_backward(ocfd_mlp* n, const float* T, long long M, cudaStream_t st, int nblk_loss) {
-    const int sms = n->ctx->num_sms;
-    const int ntile = (int)(M / 128), nchunk = (int)(M / CHUNK);
-    k_mlp_out_grad<<<nblk_loss, 256, 0, st>>>(n->Y, T, n->dZ4, M, n->lossp);
-    const MlpNet net = net_of(n);
-    // layer 4 (output): weights from dZ4 and H4
-    k_mlp_bwd_weight<<<nchunk, 128, SW_TOT, st>>>(4, n->dZ4, n->H + 3LL * M * 128, 128, n->partW, n->partb,
-                                                   n->ctx->d_error);
-    // dZ3 = (dZ4 W5) * gelu'(Z4)
-    const float* dcur = n->dZ4;
-    float* dnext = n->dZa;
-    for (int l = 4; l >= 1; --l) {
-        k_mlp_bwd_data<<<std::min(ntile, sms), 128, SD_TOT, st>>>(net, l, dcur, n->Z + (long long)(l - 1) * M * 128,
-                                                                  dnext, ntile, n->ctx->d_error);
-        // weights of layer l-1 from dZ_{l-1} and its input (H_{l-1}, or X for l-1 = 0)
-        const uint16_t* A = (l - 1 == 0) ? n->Xb : n->H + (long long)(l - 2) * M * 128;
-        k_mlp_bwd_weight<<<nchunk, 128, SW_TOT, st>>>(l - 1, dnext, A, (l - 1 == 0) ? 16 : 128, n->partW, n->partb,
-                                                       n->ctx->d_error);
-        dcur = dnext;
-        dnext = (dnext == n->dZa) ? n->dZb : n->dZa;
-    }
-    (void)sms;
+// `nblk` receives the number of partial sums in lossp
+static ocfd_status mlp_backward(ocfd_mlp* n, const float* T, long long M, cudaStream_t st, int& nblk) {
+    const int ntile = (int)(M / 128);
+    nblk = std::min(ntile, n->ctx->num_sms);
+    k_mlp_bwd<<<nblk, MLP_THREADS, SD_TOT, st>>>(n->Wt, n->Y, T, n->Z, n->dZ4, n->dZ, n->lossp, ntile, n->ctx->d_error);
+    k_mlp_bwd_weight<<<dim3((unsigned)(M / CHUNK), 5), WG_THREADS, SW_TOT, st>>>(n->dZ4, n->dZ, n->Xb, n->H, M, n->partW,
+                                                                              n->partb, n->ctx->d_error);
     return check_launch("MLP backward");
 }
 
@@ -431,7 +513,7 @@ using namespace ocfd;
 extern "C" {
 
 ocfd_status ocfd_mlp_create(ocfd_context* ctx, int32_t max_batch, uint64_t seed, ocfd_mlp** out) {
-    if (!ctx || !out || max_batch < CHUNK || max_batch % CHUNK)
+    if (!ctx || !out || max_batch < BATCH_ROWS || max_batch % BATCH_ROWS)
         return fail(OCFD_BAD_ARG, "ocfd_mlp_create: max_batch must be a positive multiple of 256");
     *out = nullptr;
     ocfd_status s = mlp_configure();
@@ -452,13 +534,13 @@ ocfd_status ocfd_mlp_create(ocfd_context* ctx, int32_t max_batch, uint64_t seed,
     al((void**)&n->mb, 4 * BTOT);
     al((void**)&n->vb, 4 * BTOT);
     al((void**)&n->Wb, 2 * WTOT);
+    al((void**)&n->Wt, 2 * WTOT);
     al((void**)&n->Xb, 2 * M * 16);
     al((void**)&n->Y, 4 * M * 16);
     al((void**)&n->Z, 4 * 4 * M * 128);
     al((void**)&n->H, 2 * 4 * M * 128);
     al((void**)&n->dZ4, 4 * M * 16);
-    al((void**)&n->dZa, 4 * M * 128);
-    al((void**)&n->dZb, 4 * M * 128);
+    al((void**)&n->dZ, 4 * 4 * M * 128);
     al((void**)&n->partW, 4 * nchunk * WTOT);
     al((void**)&n->partb, 4 * nchunk * BTOT);
     al((void**)&n->lossp, 4 * 1024);
@@ -489,7 +571,7 @@ ocfd_status ocfd_mlp_create(ocfd_context* ctx, int32_t max_batch, uint64_t seed,
     for (int i = 0; i < MLP_IN; ++i) n->norm[MLP_IN + i] = 1.0f;
     for (int i = 0; i < MLP_OUT; ++i) n->norm[2 * MLP_IN + MLP_OUT + i] = 1.0f;
     cudaMemcpy(n->W32, W.data(), 4 * WTOT, cudaMemcpyHostToDevice);
-    k_mlp_to_bf16<<<64, 256>>>(n->W32, n->Wb);
+    k_mlp_to_bf16<<<64, 256>>>(n->W32, n->Wb, n->Wt);
     s = check_launch("ocfd_mlp_create");
     if (s == OCFD_OK && cudaDeviceSynchronize() != cudaSuccess) s = check_launch("ocfd_mlp_create");
     if (s != OCFD_OK) {
@@ -502,8 +584,8 @@ ocfd_status ocfd_mlp_create(ocfd_context* ctx, int32_t max_batch, uint64_t seed,
 
 ocfd_status ocfd_mlp_destroy(ocfd_mlp* n) {
     if (!n) return OCFD_OK;
-    void* ps[] = {n->W32, n->b32, n->mW, n->vW, n->mb, n->vb, n->Wb, n->Xb, n->Y, n->Z, n->H, n->dZ4, n->dZa,
-                  n->dZb, n->partW, n->partb, n->lossp, n->gW, n->gb};
+    void* ps[] = {n->W32, n->b32, n->mW, n->vW, n->mb, n->vb, n->Wb, n->Wt, n->Xb, n->Y, n->Z, n->H, n->dZ4, n->dZ,
+                  n->partW, n->partb, n->lossp, n->gW, n->gb};
     for (void* p : ps) cudaFree(p);
     delete n;
     return OCFD_OK;
@@ -542,7 +624,7 @@ ocfd_status ocfd_mlp_set_params(ocfd_mlp* n, const float* W, const float* b) {
     if ((W && cudaMemcpy(n->W32, W, 4 * WTOT, cudaMemcpyHostToDevice) != cudaSuccess) ||
         (b && cudaMemcpy(n->b32, b, 4 * BTOT, cudaMemcpyHostToDevice) != cudaSuccess))
         return check_launch("ocfd_mlp_set_params");
-    k_mlp_to_bf16<<<64, 256>>>(n->W32, n->Wb);
+    k_mlp_to_bf16<<<64, 256>>>(n->W32, n->Wb, n->Wt);
     return check_launch("ocfd_mlp_set_params");
 }
 
@@ -575,25 +657,25 @@ ocfd_status ocfd_mlp_forward(ocfd_mlp* n, const float* X, float* Y, int64_t M, v
 // only (gW [WTOT], gb [BTOT] on the host when given).  loss: host scalar.
 ocfd_status ocfd_mlp_train_step(ocfd_mlp* n, const float* X, const float* T, int64_t M, float lr, int32_t update,
                                 float* loss, float* gW, float* gb, void* stream) {
-    if (!n || !X || !T || M <= 0 || M % CHUNK || M > n->max_batch)
+    if (!n || !X || !T || M <= 0 || M % BATCH_ROWS || M > n->max_batch)
         return fail(OCFD_BAD_ARG, "ocfd_mlp_train_step: M must be a multiple of 256 up to max_batch");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     ocfd_status s = mlp_forward(n, X, M, st);
     if (s != OCFD_OK) return s;
-    const int nblk = 256;
+    int nblk = 0;
     s = mlp_backward(n, T, M, st, nblk);
     if (s != OCFD_OK) return s;
     if (update) ++n->steps;
     const float c1 = update ? (float)(1.0 / (1.0 - std::pow(0.9, (double)n->steps))) : 1.0f;
     const float c2 = update ? (float)(1.0 / (1.0 - std::pow(0.999, (double)n->steps))) : 1.0f;
     k_mlp_reduce_adam<<<grid_for(WTOT + BTOT, 256, n->ctx->num_sms), 256, 0, st>>>(
-        n->partW, n->partb, (int)(M / CHUNK), n->W32, n->b32, n->mW, n->vW, n->mb, n->vb, n->Wb, n->gW, n->gb, lr, c1,
+        n->partW, n->partb, (int)(M / CHUNK), n->W32, n->b32, n->mW, n->vW, n->mb, n->vb, n->Wb, n->Wt, n->gW, n->gb, lr, c1,
         c2, update);
     s = check_launch("ocfd_mlp_train_step");
     if (s != OCFD_OK) return s;
     if (loss) {
-        float lp[nblk];
-        if (cudaMemcpyAsync(lp, n->lossp, sizeof(lp), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+        float lp[1024];
+        if (cudaMemcpyAsync(lp, n->lossp, sizeof(float) * nblk, cudaMemcpyDeviceToHost, st) != cudaSuccess)
             return check_launch("ocfd_mlp_train_step");
         s = mlp_check_error(n, st, "ocfd_mlp_train_step");
         if (s != OCFD_OK) return s;
