@@ -140,41 +140,37 @@ __device__ __forceinline__ double rcp_nr(double x) {
 // i+2..i-2, i.e. wenoz_minus(V1..V5) == wenoz_1rcp(V5, V4, V3, V2, V1)).  With
 // the first differences d1..d4 of V1..V5 and the second differences e1 = d2 - d1,
 // e2 = d3 - d2, e3 = d4 - d3:
-//   - The smoothness indicators (13/12) e^2 + (1/4) g^2 are positive definite forms
-//     of one first and one second difference, beta_1 = d2^2 + e1 (d2 + 4/3 e1),
-//     beta_2 = d2^2 + e2 (d2 + 4/3 e2), beta_3 = d3^2 + e3 (4/3 e3 - d3).
-//   - The weights alpha_k = c_k (1 + (tau / D_k)^2), D_k = eps + beta_k, c = (1, 6,
-//     3), are multiplied by the common positive factor (D_1 D_2 D_3)^2, which
-//     cancels in alpha_k / sum alpha: with q_k = D_k^2, alpha_k becomes c_k A_k,
-//     A_k = q_j q_l (q_k + tau^2) ({j, l} the other two), formed on the integer
-//     pipes (weno_weights.cuh).
+//   - The smoothness indicators are (13/12) e_k^2 + (1/4) g_k^2 with g_1 = 2 d2 + e1,
+//     g_2 = d2 + d3, g_3 = 2 d3 - e3; the weights alpha_k = c_k (1 + (tau / D_k)^2),
+//     D_k = eps + beta_k, c = (1, 6, 3), are multiplied by the common positive factor
+//     (D_1 D_2 D_3)^2, which cancels in alpha_k / sum alpha: with q_k = D_k^2, alpha_k
+//     becomes c_k A_k, A_k = q_j q_l (q_k + tau^2) ({j, l} the other two).  All of this
+//     is done on the integer pipes (weno_weights.cuh).
 //   - The candidate polynomials are V3 + (3 d2 + 2 e1) / 6, V3 + (3 d2 + 2 e2) / 6
 //     and V3 + (3 d2 + 3 e2 - e3) / 6, so the face value is
 //     V3 + d2 / 2 + (2 A_1 e1 + 12 A_2 e2 + 3 A_3 (3 e2 - e3)) / (6 sum c_k A_k):
 //     three products, and the rounding of the weights multiplies second
 //     differences only.
 // The same value up to rounding (parity tests: 1e-12 per right-hand side), finite
-// for flux differences below ~1e150.  Differences, and S = eps + d^2, belong to
-// cells of the line and serve neighbouring faces: 18.5 FP64 operations per face
-// and side in runs of three faces (24 for a face alone).  With indicators and
-// candidates formed from the values and all of it in FP64 they were 49 (54), and a
-// stage of the 3D blast on 128x128x64 cells took 4.00 ms; this way 2.17 ms.
+// for flux differences below ~1e150.  Differences and curvature terms belong to
+// cells of the line and serve neighbouring faces: 13 FP64 operations per face and
+// side in runs of three faces (17 for a face alone).  With indicators and candidates
+// formed from the values and all of it in FP64 they were 49 (54), and a stage of the
+// 3D blast on 128x128x64 cells took 4.00 ms; this way 1.91 ms.
 // Every rounding is written out, so the value does not depend on the code around
 // the call.
-__device__ __forceinline__ double wenoz_s(double d) { return __fma_rn(d, d, 1e-6); }
 __device__ __forceinline__ double wenoz_face_d(double V3, double d2, double d3, double e1, double e2, double e3,
-                                               double S2, double S3) {
-    const double D1 = __fma_rn(e1, __fma_rn(4.0 / 3.0, e1, d2), S2);
-    const double D2 = __fma_rn(e2, __fma_rn(4.0 / 3.0, e2, d2), S2);
-    const double D3 = __fma_rn(e3, __fma_rn(4.0 / 3.0, e3, -d3), S3);
+                                               const wz::Num& k1, const wz::Num& k2, const wz::Num& k3) {
+    const double g1 = __fma_rn(2.0, d2, e1), g2 = __dadd_rn(d2, d3), g3 = __fma_rn(2.0, d3, -e3);
     double c1, c2, c3;
-    wz::weights(D1, D2, D3, fabs(__dsub_rn(D1, D3)), c1, c2, c3);
+    wz::weights(g1, g2, g3, k1, k2, k3, c1, c2, c3);
     const double corr = __fma_rn(c3, __fma_rn(3.0, e2, -e3), __fma_rn(c2, e2, __dmul_rn(c1, e1)));
     return __dadd_rn(__fma_rn(0.5, d2, V3), corr);
 }
 __device__ __forceinline__ double wenoz_1rcp(double V1, double V2, double V3, double V4, double V5) {
     const double d1 = __dsub_rn(V2, V1), d2 = __dsub_rn(V3, V2), d3 = __dsub_rn(V4, V3), d4 = __dsub_rn(V5, V4);
-    return wenoz_face_d(V3, d2, d3, __dsub_rn(d2, d1), __dsub_rn(d3, d2), __dsub_rn(d4, d3), wenoz_s(d2), wenoz_s(d3));
+    const double e1 = __dsub_rn(d2, d1), e2 = __dsub_rn(d3, d2), e3 = __dsub_rn(d4, d3);
+    return wenoz_face_d(V3, d2, d3, e1, e2, e3, wz::curvature(e1), wz::curvature(e2), wz::curvature(e3));
 }
 // one side of faces m = 0, 1, 2 whose stencils (ordered towards the face) are
 // a[m s] .. a[(m + 4) s], as a window sliding along the line.  The f+ side of a
@@ -186,10 +182,10 @@ __device__ __forceinline__ void wenoz_run3(const double* a, int s, double& o0, d
     const double V2 = a[s], d1 = __dsub_rn(V2, a[0]);
     double d2 = __dsub_rn(V3, V2), d3 = __dsub_rn(V4, V3), d4 = __dsub_rn(V5, V4);
     double e1 = __dsub_rn(d2, d1), e2 = __dsub_rn(d3, d2), e3 = __dsub_rn(d4, d3);
-    double S2 = wenoz_s(d2), S3 = wenoz_s(d3);
+    wz::Num k1 = wz::curvature(e1), k2 = wz::curvature(e2), k3 = wz::curvature(e3);
 #pragma unroll 1
     for (int m = 0; m < 3; ++m) {
-        const double v = wenoz_face_d(V3, d2, d3, e1, e2, e3, S2, S3);
+        const double v = wenoz_face_d(V3, d2, d3, e1, e2, e3, k1, k2, k3);
         if (m == 0) o0 = v;
         else if (m == 1) o1 = v;
         else o2 = v;
@@ -203,8 +199,9 @@ __device__ __forceinline__ void wenoz_run3(const double* a, int s, double& o0, d
             e1 = e2;
             e2 = e3;
             e3 = __dsub_rn(d4, d3);
-            S2 = S3;
-            S3 = wenoz_s(d3);
+            k1 = k2;
+            k2 = k3;
+            k3 = wz::curvature(e3);
         }
     }
 }

@@ -63,7 +63,6 @@ struct Pencil {
     static constexpr int NF = FX * FY * FZ;
     static constexpr int PST = D == 0 ? 1 : (D == 1 ? PX : PX * PY);  // pencil stride along D
     static constexpr int FST = D == 0 ? 1 : (D == 1 ? FX : FX * FY);  // face stride along D
-    static constexpr int SMEM = 10 * N + 5 * NF;                       // elements
 };
 
 // threads of a tile's CTA: one per cell, and in small tiles enough for the WENO-Z
@@ -81,12 +80,18 @@ struct Ring {
     static constexpr int N = RX * RY * RZ;
 };
 
+// The split pencils (10 values per cell) and, behind the longest of them, the face
+// fluxes (5 per face): at one place for the three sweeps, so that a sweep's cells can
+// be split while the last one's face fluxes are still read.
+__host__ __device__ constexpr int max3(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
+template <int TX, int TY, int TZ>
+__host__ __device__ constexpr int face_offset() {
+    return 10 * max3(Pencil<0, TX, TY, TZ>::N, Pencil<1, TX, TY, TZ>::N, Pencil<2, TX, TY, TZ>::N);
+}
 template <int TX, int TY, int TZ>
 __host__ __device__ constexpr int pencil_elems() {
-    constexpr int a = Pencil<0, TX, TY, TZ>::SMEM;
-    constexpr int b = Pencil<1, TX, TY, TZ>::SMEM;
-    constexpr int c = Pencil<2, TX, TY, TZ>::SMEM;
-    return a > b ? (a > c ? a : c) : (b > c ? b : c);
+    return face_offset<TX, TY, TZ>() +
+           5 * max3(Pencil<0, TX, TY, TZ>::NF, Pencil<1, TX, TY, TZ>::NF, Pencil<2, TX, TY, TZ>::NF);
 }
 
 // tiles whose cross is staged by TMA (see the file comment): the staged
@@ -601,7 +606,8 @@ __device__ __forceinline__ void sweep(const RegBoxArgs& B, const DevParm& P, int
             }
         }
     }
-    __syncthreads();
+    // no barrier here: the next sweep writes the split pencil, which nothing reads any
+    // more, and its face fluxes only behind its first barrier
 }
 
 // One tile (index t over the box list, or over the single box) of the fused
@@ -669,17 +675,17 @@ __device__ __forceinline__ void rhs_tile(const RegBoxArgs* __restrict__ boxes, c
         cross_prims<TX, TY, TZ>(B, P, i0, j0, k0, stage, staged, Q);
         __syncthreads();
         FT* F = reinterpret_cast<FT*>(sbase);
-        sweep<FT, 0, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + 10 * Pencil<0, TX, TY, TZ>::N, nullptr, acc, Q);
-        sweep<FT, 1, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + 10 * Pencil<1, TX, TY, TZ>::N, nullptr, acc, Q);
-        sweep<FT, 2, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + 10 * Pencil<2, TX, TY, TZ>::N, nullptr, acc, Q);
+        sweep<FT, 0, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), nullptr, acc, Q);
+        sweep<FT, 1, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), nullptr, acc, Q);
+        sweep<FT, 2, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), nullptr, acc, Q);
     } else if constexpr (CrossPlain<FT, TX, TY, TZ, VISC>::value) {
         FT* F = reinterpret_cast<FT*>(sbase);
         double* Q = F + pencil_elems<TX, TY, TZ>();
         cross_prims_plain<TX, TY, TZ>(B, P, i0, j0, k0, Q);
         __syncthreads();
-        sweep<FT, 0, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + 10 * Pencil<0, TX, TY, TZ>::N, nullptr, acc, Q);
-        sweep<FT, 1, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + 10 * Pencil<1, TX, TY, TZ>::N, nullptr, acc, Q);
-        sweep<FT, 2, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + 10 * Pencil<2, TX, TY, TZ>::N, nullptr, acc, Q);
+        sweep<FT, 0, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), nullptr, acc, Q);
+        sweep<FT, 1, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), nullptr, acc, Q);
+        sweep<FT, 2, TX, TY, TZ, VISC, true>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), nullptr, acc, Q);
     } else {
     constexpr int PMAX = pencil_elems<TX, TY, TZ>();
     FT* smem = reinterpret_cast<FT*>(sbase);
@@ -705,9 +711,9 @@ __device__ __forceinline__ void rhs_tile(const RegBoxArgs* __restrict__ boxes, c
         }
         __syncthreads();
     }
-    sweep<FT, 0, TX, TY, TZ, VISC>(B, P, i0, j0, k0, F, F + 10 * Pencil<0, TX, TY, TZ>::N, ring, acc);
-    sweep<FT, 1, TX, TY, TZ, VISC>(B, P, i0, j0, k0, F, F + 10 * Pencil<1, TX, TY, TZ>::N, ring, acc);
-    sweep<FT, 2, TX, TY, TZ, VISC>(B, P, i0, j0, k0, F, F + 10 * Pencil<2, TX, TY, TZ>::N, ring, acc);
+    sweep<FT, 0, TX, TY, TZ, VISC>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), ring, acc);
+    sweep<FT, 1, TX, TY, TZ, VISC>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), ring, acc);
+    sweep<FT, 2, TX, TY, TZ, VISC>(B, P, i0, j0, k0, F, F + face_offset<TX, TY, TZ>(), ring, acc);
     }
 
     const int ti = threadIdx.x % TX, tj = (threadIdx.x / TX) % TY, tk = threadIdx.x / (TX * TY);

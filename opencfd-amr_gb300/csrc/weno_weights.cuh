@@ -3,18 +3,20 @@
 // GB300 executes two FP64 instructions per cycle per SM and 64 to 128 integer
 // instructions, so a product of positive numbers as 64-bit integers with separate
 // exponents (three 32 x 32 -> 64 bit multiply-adds, a shift and an add) costs a
-// fraction of one FP64 multiplication's issue time.  The weights are sums and
-// products of positive numbers only.  Values are m 2^e with m below 2^63 and
-// truncated products, between 55 and 62 significant bits at every step against
-// FP64's 53, and the division is one by the sum's integer reciprocal: the results
-// are rounded to FP64 once.  Largest relative error 1.5e-16 (rms 0.5e-16) against
-// 7.5e-16 (1.1e-16) for the same weights in FP64 arithmetic.  Exponents are
+// fraction of one FP64 multiplication's issue time.  The smoothness indicators are
+// sums of two squares and the weights sums and products of them.  Values are m 2^e
+// with m below 2^63 and truncated products, between 54 and 62 significant bits at
+// every step against FP64's 53, and the division is one by the sum's integer
+// reciprocal: the results are rounded to FP64 once.  Against 128-bit arithmetic the
+// coefficients' error is 0.5e-16 rms, where the same formulas in FP64 have 0.8e-16 to
+// 6e-16; where tau cancels both lose digits, this form six bits fewer.  Exponents are
 // integers, so no intermediate overflows or underflows.
-// It replaces 19 of the 37 FP64 operations of a face and side by about 250 integer
-// ones, which run in the FP64 pipe's shadow: a stage of the 3D blast on 128x128x64
-// cells 3.32 -> 2.17 ms, the FP64 pipe 82 % busy with 1022 instead of 1630
-// instructions per cell and the SM issuing 0.88 instead of 0.37 instructions per
-// cycle.  (With the sum's reciprocal and the division in FP64: 2.38 ms.)
+// They replace 24 of 37 FP64 operations of a face and side by about 400 integer
+// instructions, which run in the FP64 pipe's shadow.  A stage of the 3D blast on
+// 128x128x64 cells: 3.32 ms in FP64; 2.38 ms with the weights here; 2.17 ms with
+// the division too; 1.91 ms with the indicators too (808 instead of 1630 FP64
+// instructions per cell, the FP64 pipe 74 % busy, 1.26 instead of 0.37 instructions
+// issued per cycle).
 #pragma once
 
 #include <cstdint>
@@ -81,21 +83,15 @@ struct Num {  // m 2^e
     uint64_t m;
     int e;
 };
-// a positive double: m in [2^62, 2^63), e its biased exponent (a zero or denormal
-// becomes about 2^-1023, far below every square it is added to)
-OCFD_HD Num unpack(double x) {
-    const uint64_t b = bits_of(x);
-    return Num{((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10, (int)(b >> 52)};
-}
-// m >= 2^32 shifted up to [2^63, 2^64)
+// m in [2^32, 2^63) shifted up to [2^62, 2^63)
 OCFD_HD Num normalise(uint64_t m, int e) {
-    const int z = lead_zeros((uint32_t)(m >> 32));
+    const int z = lead_zeros((uint32_t)(m >> 32)) - 1;
     return Num{m << z, e - z};
 }
-// the double nearest m 2^e (m in [2^63, 2^64)), at least 2^-1022
+// the double nearest m 2^e (m in [2^62, 2^63)), at least 2^-1022
 OCFD_HD double pack(const Num& a) {
-    const int x = imax(a.e + 63 + 1022, 0);  // biased exponent - 1: the leading bit adds one
-    return double_of((a.m >> 11) + ((a.m >> 10) & 1u) + ((uint64_t)(uint32_t)x << 52));
+    const int x = imax(a.e + 62 + 1022, 0);  // biased exponent - 1: the leading bit adds one
+    return double_of(((a.m + 0x200u) >> 10) + ((uint64_t)(uint32_t)x << 52));
 }
 // about 1/x to FP32 accuracy (the seed below corrects any error up to 2^-20)
 OCFD_HD float rcp_seed(float x) {
@@ -107,9 +103,10 @@ OCFD_HD float rcp_seed(float x) {
     return 1.0f / x;
 #endif
 }
-// 2^126 / m to within a few units, below 2^63 (m in [2^63, 2^64)): an FP32 seed y of
+// 2^125 / m to within a few units, below 2^63 (m in [2^62, 2^63)): an FP32 seed y of
 // relative error e <= 2^-20 and one cubic step y (1 + e + e^2)
 OCFD_HD uint64_t recip(uint64_t m) {
+    m *= 2;
     const uint32_t mh = (uint32_t)(m >> 32), ml = (uint32_t)m;
     const uint32_t y = (uint32_t)(rcp_seed((float)mh) * 0x1p62f);         // (2^30, 2^31]
     const uint64_t t = (uint64_t)mh * y + (((uint64_t)ml * y) >> 32);     // 2^62 (1 - e)
@@ -121,11 +118,44 @@ OCFD_HD uint64_t recip(uint64_t m) {
     return ((uint64_t)y << 32) + (uint64_t)(((int64_t)ch * (int64_t)y) >> 8) + (((uint64_t)cl * y) >> 30) - 8;
 }
 
-// The WENO-Z correction's coefficients: from D_k = eps + beta_k > 0 and tau = |D_1 -
-// D_3|, with q_k = D_k^2, A_k = q_i q_j (q_k + tau^2) ({i, j} the other two) and s =
-// A_1 + 6 A_2 + 3 A_3: c1 = A_1 / (3 s), c2 = 6 A_2 / (3 s), c3 = 3 A_3 / (6 s).
-OCFD_HD void weights(double D1, double D2, double D3, double tau, double& c1, double& c2, double& c3) {
-    const Num d1 = unpack(D1), d2 = unpack(D2), d3 = unpack(D3), t = unpack(tau);
+// |x| as a square's factor: m in [2^62, 2^63), biased exponent
+OCFD_HD Num unpack_abs(double x) {
+    const uint64_t b = bits_of(x) & 0x7fffffffffffffffull;
+    return Num{((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10, (int)(b >> 52)};
+}
+// Squares stand for m 2^(e - 2106) here.  12 eps + 13 e^2 of a second difference e,
+// the part of 12 (eps + beta) that belongs to a triple of cells (eps = 1e-6)
+constexpr uint64_t kEps12 = 0x192a737110e45380ull;  // 12 eps = kEps12 2^-77
+constexpr int kEps12Exp = 2106 - 77;
+OCFD_HD Num curvature(double e) {
+    const Num a = unpack_abs(e);
+    const int x = 2 * a.e + 5;
+    return Num{shr((sq_hi(a.m) >> 5) * 13, imax(kEps12Exp - x, 0)) + shr(kEps12, imax(x - kEps12Exp, 0)),
+               imax(x, kEps12Exp)};  // [2^58, 2^62)
+}
+// D = 12 (eps + beta) = 3 g^2 + (12 eps + 13 e^2), m in [2^62, 2^63)
+OCFD_HD Num indicator(double g, const Num& c) {
+    const Num a = unpack_abs(g);
+    const int x = 2 * a.e + 2;
+    return normalise(shr((sq_hi(a.m) >> 2) * 3, imax(c.e - x, 0)) + shr(c.m, imax(x - c.e, 0)), imax(x, c.e));
+}
+// |a - b|, m in [2^62, 2^63) or 0
+OCFD_HD Num difference(const Num& a, const Num& b) {
+    const int x = imax(a.e, b.e);
+    const int64_t d = (int64_t)(shr(a.m, x - a.e) - shr(b.m, x - b.e));
+    const uint64_t m = (uint64_t)(d < 0 ? -d : d);
+    const int z = ((m >> 32) ? lead_zeros((uint32_t)(m >> 32)) : 32 + lead_zeros((uint32_t)m | 1u)) - 1;
+    return Num{m << z, x - z};
+}
+
+// The WENO-Z correction's coefficients: with D_k = 12 (eps + beta_k) from the first
+// differences g_k = 2 sqrt(beta_k - 13/12 e_k^2) and the curvature terms of the three
+// sub-stencils, tau = |D_1 - D_3|, q_k = D_k^2, A_k = q_i q_j (q_k + tau^2) ({i, j} the
+// other two) and s = A_1 + 6 A_2 + 3 A_3: c1 = A_1 / (3 s), c2 = 6 A_2 / (3 s), c3 =
+// 3 A_3 / (6 s).
+OCFD_HD void weights(double g1, double g2, double g3, const Num& k1, const Num& k2, const Num& k3, double& c1,
+                     double& c2, double& c3) {
+    const Num d1 = indicator(g1, k1), d2 = indicator(g2, k2), d3 = indicator(g3, k3), t = difference(d1, d3);
     const uint64_t q1 = sq_hi(d1.m), q2 = sq_hi(d2.m), q3 = sq_hi(d3.m), tt = sq_hi(t.m);  // [2^60, 2^62)
     const int e1 = 2 * d1.e, e2 = 2 * d2.e, e3 = 2 * d3.e, et = 2 * t.e;
     // q_k + tau^2 at the larger exponent
@@ -135,15 +165,15 @@ OCFD_HD void weights(double D1, double D2, double D3, double tau, double& c1, do
     const uint64_t r23 = mul_hi(2 * q2, 2 * q3) * 2, r13 = mul_hi(2 * q1, 2 * q3) * 2, r12 = mul_hi(2 * q1, 2 * q2) * 2;
     // A_k in [2^55, 2^62); the constant exponent offsets are common to all three
     const Num b1 = normalise(mul_hi(r23, s1), e2 + e3 + imax(e1, et));
-    const Num b2 = normalise(3 * mul_hi(r13, s2), e1 + e3 + imax(e2, et) + 1);  // 6 A_2
-    const Num b3 = normalise(3 * mul_hi(r12, s3), e1 + e2 + imax(e3, et));      // 3 A_3
+    const Num b2 = normalise(3 * (mul_hi(r13, s2) >> 1), e1 + e3 + imax(e2, et) + 2);  // 6 A_2
+    const Num b3 = normalise(3 * (mul_hi(r12, s3) >> 1), e1 + e2 + imax(e3, et) + 1);  // 3 A_3
     const int top = imax(b1.e, imax(b2.e, b3.e)) + 4;
     const Num s = normalise(3 * (shr(b1.m, top - b1.e) + shr(b2.m, top - b2.e) + shr(b3.m, top - b3.e)), top);  // 3 s
     const uint64_t z = recip(s.m);
-    // b / (3 s) = (b.m / 2) z 2^-61 2^(b.e - s.e)
-    c1 = pack(normalise(mul_hi(b1.m >> 1, z), b1.e - s.e - 61));
-    c2 = pack(normalise(mul_hi(b2.m >> 1, z), b2.e - s.e - 61));
-    c3 = pack(normalise(mul_hi(b3.m >> 1, z), b3.e - s.e - 62));
+    // b / (3 s) = b.m z 2^-125 2^(b.e - s.e)
+    c1 = pack(normalise(mul_hi(b1.m, z), b1.e - s.e - 61));
+    c2 = pack(normalise(mul_hi(b2.m, z), b2.e - s.e - 61));
+    c3 = pack(normalise(mul_hi(b3.m, z), b3.e - s.e - 62));
 }
 
 }  // namespace wz

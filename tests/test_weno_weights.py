@@ -18,67 +18,73 @@ def weights(tmp_path_factory):
     d = tmp_path_factory.mktemp("wz")
     src, so = d / "wz.cpp", d / "wz.so"
     src.write_text('#include "weno_weights.cuh"\n'
-                   'extern "C" void w(const double* D, double* c) '
-                   '{ ocfd::wz::weights(D[0], D[1], D[2], D[3], c[0], c[1], c[2]); }\n')
+                   'using namespace ocfd::wz;\n'
+                   'extern "C" void w(const double* g, const double* e, double* c) '
+                   '{ weights(g[0], g[1], g[2], curvature(e[0]), curvature(e[1]), curvature(e[2]), c[0], c[1], c[2]); }\n')
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(so)], check=True)
     lib = ctypes.CDLL(str(so))
 
-    def f(D1, D2, D3, tau):
-        a, c = (ctypes.c_double * 4)(D1, D2, D3, tau), (ctypes.c_double * 3)()
-        lib.w(a, c)
+    def f(g, e):
+        c = (ctypes.c_double * 3)()
+        lib.w((ctypes.c_double * 3)(*g), (ctypes.c_double * 3)(*e), c)
         return list(c)
     return f
 
 
-def exact_coefficients(D, tau):
-    q, t = [Q(x) ** 2 for x in D], Q(tau) ** 2
+def exact_coefficients(g, e):
+    D = [Q(1e-6) + Q(x) ** 2 / 4 + Q(13, 12) * Q(y) ** 2 for x, y in zip(g, e)]
+    q, t = [x ** 2 for x in D], (D[0] - D[2]) ** 2
     A = [q[1] * q[2] * (q[0] + t), q[0] * q[2] * (q[1] + t), q[0] * q[1] * (q[2] + t)]
     s = A[0] + 6 * A[1] + 3 * A[2]
-    return [A[0] / (3 * s), 2 * A[1] / s, A[2] / (2 * s)]
+    # the error of tau, the difference of two indicators within 2^-55, in the weights
+    d = Q(2) ** -55 * max(D[0], D[2])
+    amp = max((2 * abs(D[0] - D[2]) * d + d * d) / (x + t) for x in q)
+    return [A[0] / (3 * s), 2 * A[1] / s, A[2] / (2 * s)], amp
 
 
-# Relative error bound, in units of 2^-53: a product of two numbers below 2^63 keeps
-# at least 55 bits and is truncated by less than 2, so A_k and the sum are each
-# within 0.8; the reciprocal and the last products add less than 0.1; the rounding 1.
-TOL = 3 * 2.0 ** -53
+# Relative error bound.  An indicator is a sum of two squares, each truncated by less
+# than 2^-55; the weights take it to at most the fourth power; tau's error is the
+# indicators' and is followed exactly (amp: FP64 arithmetic has eight times as much).
+# A product keeps at least 55 bits and is truncated by less than 2, so A_k and the
+# sum add 0.8 units of 2^-53 each, the reciprocal and the last products less than
+# 0.1, the rounding 1.
+TOL = 4 * 2.0 ** -53
 
 
-@pytest.mark.parametrize("lo,hi", [(-6, -5.99), (-6, 0), (-6, 10), (-3, 45), (40, 50)])
+@pytest.mark.parametrize("lo,hi", [(-12, -6), (-3, -1), (-2, 0), (-6, 5), (-3, 22), (18, 24)])
 def test_weights_exact(weights, lo, hi):
     rng = np.random.default_rng(abs(int(100 * hi)))
     for n in range(400):
-        D = [max(1e-6, float(x)) for x in 10.0 ** rng.uniform(lo, hi, 3)]
+        g, e = [[float(x) for x in 10.0 ** rng.uniform(lo, hi, 3) * rng.choice([-1, 1], 3)] for _ in range(2)]
         if n % 5 == 1:
-            D[2] = D[0] * (1 + 2.0 ** -40 * rng.standard_normal())
+            g[2], e[2] = g[0] * (1 + 2.0 ** -40 * rng.standard_normal()), -e[0]
         if n % 5 == 2:
-            D[1] = D[2] = D[0]
+            g[1] = g[2] = g[0]
+            e[1] = e[2] = e[0]
         if n % 5 == 3:  # powers of two and their neighbours: every carry of the mantissas
-            D = [float(np.nextafter(2.0 ** np.ceil(np.log2(x)), rng.choice([0.0, 1e300]))) for x in D]
-            D = [max(1e-6, x) for x in D]
-        tau = abs(D[0] - D[2])
-        for got, want in zip(weights(*D, tau), exact_coefficients(D, tau)):
-            if want > Q(2) ** -1000:
-                assert abs(Q(got) - want) <= Q(TOL) * want
-            else:
+            g = [float(np.nextafter(2.0 ** np.ceil(np.log2(abs(x))), rng.choice([0.0, 1e300]))) for x in g]
+        if n % 5 == 4:
+            g[n % 3], e[(n + 1) % 3] = 0.0, 0.0
+        want, amp = exact_coefficients(g, e)
+        for got, w in zip(weights(g, e), want):
+            if w < Q(2) ** -1000:
                 assert 0 <= got <= 2.0 ** -999
+            else:
+                assert abs(Q(got) - w) <= (Q(TOL) + 2 * amp) * w
 
 
-def test_weights_smooth(weights):
-    # tau = 0 and denormal tau: the linear weights
-    for tau in (0.0, 5e-324, 1e-310):
-        c = weights(1e-6, 1e-6, 1e-6, tau)
+def test_weights_flat(weights):
+    # zero and denormal differences: the linear weights
+    for x in (0.0, 5e-324, 1e-310, 1e-200):
+        c = weights([x, -x, 0.0], [x, 0.0, -x])
         assert np.allclose(c, [1 / 30, 6 / 30, 3 / 60], rtol=2 ** -52, atol=0)
 
 
 def face(weights, V):
     d = [V[i + 1] - V[i] for i in range(4)]
     e = [d[i + 1] - d[i] for i in range(3)]
-    S = [1e-6 + x * x for x in d]
-    D1 = e[0] * (4 / 3 * e[0] + d[1]) + S[1]
-    D2 = e[1] * (4 / 3 * e[1] + d[1]) + S[1]
-    D3 = e[2] * (4 / 3 * e[2] - d[2]) + S[2]
-    c = weights(D1, D2, D3, abs(D1 - D3))
-    return (V[2] + 0.5 * d[1]) + (c[0] * e[0] + c[1] * e[1] + c[2] * (3 * e[2 - 1] - e[2]))
+    c = weights([2 * d[1] + e[0], d[1] + d[2], 2 * d[2] - e[2]], e)
+    return (V[2] + 0.5 * d[1]) + (c[0] * e[0] + c[1] * e[1] + c[2] * (3 * e[1] - e[2]))
 
 
 def face_exact(V):
