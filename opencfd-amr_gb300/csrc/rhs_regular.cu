@@ -16,6 +16,19 @@ ocfd_status configure_rhs_regular() { return configure_all<double>(); }
 
 bool regular_tile_fits(int tile, bool visc) { return tile_fits<double>(tile, visc); }
 
+// whether an SM holds two CTAs of the FP64 tile
+static bool regular_tile_pairs(int tile, bool visc) {
+    switch (tile) {
+#define OCFD_PAIRS(I, X, Y, Z, XS)                                                              \
+    case I:                                                                                     \
+        return visc ? regular_min_blocks<double, X, Y, Z, true, false>() > 1                    \
+                    : regular_min_blocks<double, X, Y, Z, false, false>() > 1;
+        OCFD_REGULAR_TILES(OCFD_PAIRS)
+#undef OCFD_PAIRS
+    }
+    return false;
+}
+
 const TileShape kRegularTiles[] = {{8, 8, 8, 0},  {8, 8, 4, 0}, {16, 8, 4, 0}, {16, 16, 2, 0}, {32, 8, 2, 0},
                                    {16, 8, 2, 0}, {8, 8, 8, 1}, {8, 8, 4, 1}, {16, 8, 4, 1}, {8, 4, 4, 0}, {4, 4, 4, 0},  {4, 4, 2, 0}};
 const int kNumRegularTiles = sizeof(kRegularTiles) / sizeof(kRegularTiles[0]);
@@ -35,8 +48,8 @@ ocfd_status launch_rhs_regular(int tile, bool visc, const RegBoxArgs* d_boxes,
 static double tile_work(const TileShape& s, bool visc, bool f32) {
     const int T[3] = {s.x, s.y, s.z};
     auto warps = [](int items) { return (items + 31) / 32; };
-    const double weno = f32 ? 150 : 115, split = f32 ? 70 : 41, prim = f32 ? 60 : 40, vface = f32 ? 120 : 95;
-    double w = 0;
+    const double weno = f32 ? 150 : 80, split = f32 ? 70 : 41, prim = f32 ? 60 : 25, vface = f32 ? 120 : 95;
+    double w = (f32 ? 200 : 65) * warps(T[0] * T[1] * T[2]);  // divergence and update
     int cross = T[0] * T[1] * T[2];
     for (int d = 0; d < 3; ++d) {
         const int line = T[(d + 1) % 3] * T[(d + 2) % 3], faces = T[d] + 1, pencil = (T[d] + 6) * line;
@@ -50,25 +63,34 @@ static double tile_work(const TileShape& s, bool visc, bool f32) {
     return w;
 }
 
-// Tile for a set of boxes: the shape that ends first on `sms` SMs.  The pipe that
+// Time of a tile shape over a set of boxes on `sms` SMs.  The pipe that
 // bounds a tile is shared by the CTAs of an SM, so a launch of n tiles takes
 // ceil(n / sms) tiles' work: large tiles have the least halo work per cell, small
-// ones spread a small box over more SMs and leave a shorter last wave.  Measured: a
+// ones spread a small box over more SMs and leave a shorter last wave.  FP64 tiles of
+// which an SM holds two keep its FP64 pipe busier (one's barriers are the other's
+// work: 8x8x4 has 12 % more work per cell than 8^3 and takes as long on large boxes,
+// 11 % less time on a slab of 512x64x4 cells than 16x8x4), hence the factor.  Measured: a
 // viscous FP64 box of 20x12x8 cells as six 8^3 tiles 207 us, as 60 tiles of 4x4x2
 // (then bound by the latency of three warps) 47 us; one of 13x97x5 cells 275 us
 // (with FP64 weights) and 44 us.  FP32 boxes take the pencil tiles: TMA staging of
 // the same shape is slower (a box of 128x96x64 cells 183 us staged, 158 us not; two
 // CTAs per SM against three).
-static int pick_tile(const int (*n)[3], int nbox, bool visc, bool f32, int ntile_shapes, int sms) {
+static double tile_cost(int t, const int (*n)[3], int nbox, bool visc, bool f32, int sms) {
+    const TileShape& s = kRegularTiles[t];
+    long long tiles = 0;
+    for (int b = 0; b < nbox; ++b)
+        tiles += (long long)((n[b][0] + s.x - 1) / s.x) * ((n[b][1] + s.y - 1) / s.y) * ((n[b][2] + s.z - 1) / s.z);
+    const double waves = tiles <= 4LL * sms ? (double)((tiles + sms - 1) / sms) : (double)tiles / sms + 0.5;
+    return waves * tile_work(s, visc, f32) * (!f32 && regular_tile_pairs(t, visc) ? 0.91 : 1.0);
+}
+
+int pick_regular_tile(const int n[3], bool visc, bool f32, int sms) {
+    const int one[1][3] = {{n[0], n[1], n[2]}};
     int best = 1;
     double best_cost = 1e300;
-    for (int t = 0; t < ntile_shapes; ++t) {
+    for (int t = 0; t < kNumRegularTiles; ++t) {
         if (!regular_tile_fits(t, visc) || kRegularTiles[t].staged) continue;
-        const TileShape& s = kRegularTiles[t];
-        long long tiles = 0;
-        for (int b = 0; b < nbox; ++b)
-            tiles += (long long)((n[b][0] + s.x - 1) / s.x) * ((n[b][1] + s.y - 1) / s.y) * ((n[b][2] + s.z - 1) / s.z);
-        const double cost = (double)((tiles + sms - 1) / sms) * tile_work(s, visc, f32);
+        const double cost = tile_cost(t, one, 1, visc, f32, sms);
         if (cost < best_cost * 0.999) {
             best_cost = cost;
             best = t;
@@ -77,12 +99,28 @@ static int pick_tile(const int (*n)[3], int nbox, bool visc, bool f32, int ntile
     return best;
 }
 
-int pick_regular_tile(const int n[3], bool visc, bool f32, int sms) {
-    const int one[1][3] = {{n[0], n[1], n[2]}};
-    return pick_tile(one, 1, visc, f32, kNumRegularTiles, sms);
+// A level's tile serves its FP64 and its FP32 steps: the shape with the least padded
+// work, where the FP32 form is fastest too, but 8x8x4 for 16x8x4 (slabs of at most
+// four cells) where that ends sooner in FP64; the FP32 form takes either alike.
+int pick_level_tile(const int (*n)[3], int nbox, int sms) {
+    int best = 1;
+    double best_cost = 1e300;
+    for (int t = 0; t < kNumPublicTiles; ++t) {
+        if (!regular_tile_fits(t, true) || kRegularTiles[t].staged) continue;
+        const TileShape& s = kRegularTiles[t];
+        double cost = 0;
+        for (int b = 0; b < nbox; ++b) {
+            const long long tiles = (long long)((n[b][0] + s.x - 1) / s.x) * ((n[b][1] + s.y - 1) / s.y) * ((n[b][2] + s.z - 1) / s.z);
+            cost += tiles * ((double)s.x * s.y * s.z * 3.0 + 6.0 * ((double)s.y * s.z + (double)s.x * s.z + (double)s.x * s.y));
+        }
+        if (cost < best_cost * 0.999) {
+            best_cost = cost;
+            best = t;
+        }
+    }
+    constexpr int T884 = 1, T1684 = 2;
+    return best == T1684 && tile_cost(T884, n, nbox, true, false, sms) < tile_cost(T1684, n, nbox, true, false, sms) ? T884 : best;
 }
-
-int pick_level_tile(const int (*n)[3], int nbox, int sms) { return pick_tile(n, nbox, true, false, kNumPublicTiles, sms); }
 
 void fill_regular_args(RegBoxArgs& a, const ocfd_array4* S, const ocfd_array4* dSdt,
                        const ocfd_array4* flux, const ocfd_box& bx, const double dxinv[3],

@@ -766,7 +766,8 @@ __device__ __forceinline__ void rhs_tile(const RegBoxArgs* __restrict__ boxes, c
 // measured faster than two without spills and than four with 32 registers)
 template <class FT, int TX, int TY, int TZ, bool VISC, bool XS>
 __host__ __device__ constexpr int regular_min_blocks() {
-    if (std::is_same<FT, double>::value) return 1;  // the FP64 WENO-Z runs hold a sliding window
+    if (std::is_same<FT, double>::value)  // the WENO-Z runs take up to 128 registers
+        return tile_threads<TX, TY, TZ>() <= 256 && 2 * (regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>() + 1024) <= 228 * 1024 ? 2 : 1;
     const int b = (int)((228u * 1024u) / (regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>() + 1024u));
     const int t = 2048 / tile_threads<TX, TY, TZ>();
     int m = b < t ? b : t;
