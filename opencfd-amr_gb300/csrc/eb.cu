@@ -1,15 +1,17 @@
 // Cut-cell box right-hand side (ideal gas), replacing the kernel chain of
 // EBR::eb_compute_dSdt_box (Source/EB/AdvanceBox.cpp:78-214):
 //   k_eb_prims      primitives over grow(bx, 2)               (c2prim)
-//   k_eb_faces<D>   per face: MUSCL-minmod left/right states of the 7
-//                   primitives, Van Leer flux, EB viscous flux (eb_recon_*,
-//                   eb_flux, eb_compute_visc_*), written to the face array
+//   k_eb_faces      per face (the three directions in one launch): MUSCL-minmod
+//                   left/right states of the 7 primitives, Van Leer flux, EB
+//                   viscous flux (eb_recon_*, eb_flux, eb_compute_visc_*),
+//                   written to the face array
 //   k_eb_div        per cell: cut-cell divergence with the wall flux, negated,
 //                   optional local rescale (eb_compute_div(_visc), flux_redist)
 // The reference stages ql/qr over the whole nodal box in HBM; here they live
 // in registers of the face thread.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "eb_physics.cuh"
@@ -46,7 +48,7 @@ __global__ void k_eb_prims(EbBoxArgs B, DevParm P) {
 }
 
 template <int D>
-__global__ void k_eb_faces(EbBoxArgs B, DevParm P) {
+__device__ __forceinline__ void eb_faces(const EbBoxArgs& B, const DevParm& P) {
     const int fx = B.hi[0] - B.lo[0] + 1 + (D == 0), fy = B.hi[1] - B.lo[1] + 1 + (D == 1),
               fz = B.hi[2] - B.lo[2] + 1 + (D == 2);
     const long long n = (long long)fx * fy * fz;
@@ -75,6 +77,13 @@ __global__ void k_eb_faces(EbBoxArgs B, DevParm P) {
     }
 }
 
+// the faces of direction blockIdx.y
+__global__ void k_eb_faces(EbBoxArgs B, DevParm P) {
+    if (blockIdx.y == 0) eb_faces<0>(B, P);
+    else if (blockIdx.y == 1) eb_faces<1>(B, P);
+    else eb_faces<2>(B, P);
+}
+
 // one cut-cell divergence (Source/EB/EBkernels.H:216-338), negated
 __global__ void k_eb_div(EbBoxArgs B, DevParm P) {
     const int nx = B.hi[0] - B.lo[0] + 1, ny = B.hi[1] - B.lo[1] + 1, nz = B.hi[2] - B.lo[2] + 1;
@@ -85,7 +94,6 @@ __global__ void k_eb_div(EbBoxArgs B, DevParm P) {
                   k = B.lo[2] + (int)(c / ((long long)nx * ny));
         const uint32_t f = B.flag(i, j, k);
         const double vf = B.vfrac(i, j, k);
-        const double tmp = B.dxinv[0] / vf;
         double out[5];
         if (eb_covered(f)) {
 #pragma unroll
@@ -97,6 +105,7 @@ __global__ void k_eb_div(EbBoxArgs B, DevParm P) {
                          B.dxinv[1] * (B.flux[1](i, j + 1, k, m) - B.flux[1](i, j, k, m)) +
                          B.dxinv[2] * (B.flux[2](i, j, k + 1, m) - B.flux[2](i, j, k, m));
         } else {
+            const double tmp = B.dxinv[0] / vf;
             const double axm = B.ap[0](i, j, k), axp = B.ap[0](i + 1, j, k);
             const double aym = B.ap[1](i, j, k), ayp = B.ap[1](i, j + 1, k);
             const double azm = B.ap[2](i, j, k), azp = B.ap[2](i, j, k + 1);
@@ -141,12 +150,10 @@ __global__ void k_eb_div(EbBoxArgs B, DevParm P) {
 #pragma unroll
             for (int m = 0; m < 5; ++m) out[m] += fw[m] * tmp;
         }
-        const bool rescale = B.redist && vf < 0.5 && vf > 0.0;
+        const long long ivf = __double_as_longlong(vf);  // 0 < vf < 0.5
+        const bool rescale = B.redist && ivf > 0 && ivf < 0x3fe0000000000000LL;
 #pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            const double divc = out[m] * -1.0;
-            B.dsdt(i, j, k, m) = rescale ? vf * divc : divc;
-        }
+        for (int m = 0; m < 5; ++m) B.dsdt(i, j, k, m) = rescale ? -(vf * out[m]) : -out[m];
     }
 }
 
@@ -235,9 +242,8 @@ static ocfd_status eb_box_launch(const char* who, ocfd_context* ctx, const ocfd_
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int T = 256, sms = ctx->num_sms;
     k_eb_prims<<<blocks_for(plan.gcells, T, sms), T, 0, st>>>(B, ctx->parm);
-    k_eb_faces<0><<<blocks_for(plan.fcells[0], T, sms), T, 0, st>>>(B, ctx->parm);
-    k_eb_faces<1><<<blocks_for(plan.fcells[1], T, sms), T, 0, st>>>(B, ctx->parm);
-    k_eb_faces<2><<<blocks_for(plan.fcells[2], T, sms), T, 0, st>>>(B, ctx->parm);
+    const long long fmax = std::max(plan.fcells[0], std::max(plan.fcells[1], plan.fcells[2]));
+    k_eb_faces<<<dim3((unsigned)blocks_for(fmax, T, sms), 3), T, 0, st>>>(B, ctx->parm);
     k_eb_div<<<blocks_for((long long)n[0] * n[1] * n[2], T, sms), T, 0, st>>>(B, ctx->parm);
     return check_launch(who);
 }
@@ -303,9 +309,7 @@ ocfd_status eb_static_scratch_resolve(ocfd_context* ctx) {
     cudaError_t e = cudaGetSymbolAddress(&p, g_eb_static_scratch);
     cudaFuncAttributes fa;
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_eb_prims);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_eb_faces<0>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_eb_faces<1>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_eb_faces<2>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_eb_faces);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_eb_div);
     if (e != cudaSuccess || !p) {
         cudaGetLastError();

@@ -523,12 +523,10 @@ __global__ void __launch_bounds__(EBT_N) k_ebl_tile(EbStageArgs A, const int* __
 #pragma unroll
                     for (int m = 0; m < 5; ++m) out[m] += fw[m] * tmp;
                 }
-                const bool rescale = A.redist && vf < 0.5 && vf > 0.0;
+                const long long ivf = __double_as_longlong(vf);  // 0 < vf < 0.5
+                const bool rescale = A.redist && ivf > 0 && ivf < 0x3fe0000000000000LL;
 #pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    const double divc = out[m] * -1.0;
-                    L[m] = rescale ? vf * divc : divc;
-                }
+                for (int m = 0; m < 5; ++m) L[m] = rescale ? -(vf * out[m]) : -out[m];
             }
         }
         double un[5];

@@ -60,6 +60,29 @@ __device__ __forceinline__ double recip<double>(double x) { return rcp_nr(x); }
 template <>
 __device__ __forceinline__ float recip<float>(float x) { return 1.0f / x; }
 
+// x >= 1, |x| < 1 and the floor of a pressure; in FP64 on the integer pipes, answering
+// as the FP64 compares do (NaN: no, no, and the floor)
+template <class T>
+__device__ __forceinline__ bool at_least_one(T x) { return x >= T(1); }
+template <class T>
+__device__ __forceinline__ bool abs_below_one(T x) { return fabs(x) < T(1); }
+template <class T>
+__device__ __forceinline__ T at_least(T x, T lo) { return x > lo ? x : lo; }
+template <>
+__device__ __forceinline__ bool at_least_one<double>(double x) {
+    const long long b = __double_as_longlong(x);
+    return b >= 0x3ff0000000000000LL && b <= 0x7ff0000000000000LL;
+}
+template <>
+__device__ __forceinline__ bool abs_below_one<double>(double x) {
+    return (__double_as_longlong(x) & 0x7fffffffffffffffLL) < 0x3ff0000000000000LL;
+}
+template <>
+__device__ __forceinline__ double at_least<double>(double x, double lo) {  // lo >= 0
+    const long long b = __double_as_longlong(x);
+    return b > __double_as_longlong(lo) && b <= 0x7ff0000000000000LL ? x : lo;
+}
+
 // Van Leer flux vector splitting, Source/EB/EBkernels.H:73-171.  The reference's
 // divisions become two reciprocals per face (the Mach numbers) and three
 // constants of gamma: rg = 1/gamma (the /gamma of the normal momentum),
@@ -71,20 +94,20 @@ template <class T>
 __device__ __forceinline__ void vanleer_g(T smallp, T gamma, T rg, T rg21, T ggm1, const T* ql, const T* qr, int D,
                                           T* flx) {
     T fp[5] = {0, 0, 0, 0, 0}, fm[5] = {0, 0, 0, 0, 0};
-    const T dl = ql[QRHO], ul = ql[QU], vl = ql[QV], wl = ql[QW], pl = ql[QPRES] > smallp ? ql[QPRES] : smallp;
-    const T dr = qr[QRHO], ur = qr[QU], vr = qr[QV], wr = qr[QW], pr = qr[QPRES] > smallp ? qr[QPRES] : smallp;
+    const T dl = ql[QRHO], ul = ql[QU], vl = ql[QV], wl = ql[QW], pl = at_least<T>(ql[QPRES], smallp);
+    const T dr = qr[QRHO], ur = qr[QU], vr = qr[QV], wr = qr[QW], pr = at_least<T>(qr[QPRES], smallp);
     const T cL = ql[QC], cR = qr[QC];
     const int nn[3] = {D == 0, D == 1, D == 2};
     const T UL = D == 0 ? ul : (D == 1 ? vl : wl);
     const T UR = D == 0 ? ur : (D == 1 ? vr : wr);
     const T ML = UL * recip<T>(cL), MR = UR * recip<T>(cR);
     const T lv[3] = {ul, vl, wl}, rv[3] = {ur, vr, wr};
-    if (ML >= T(1)) {
+    if (at_least_one<T>(ML)) {
         fp[0] = dl * UL;
 #pragma unroll
         for (int m = 0; m < 3; ++m) fp[1 + m] = dl * UL * lv[m] + T(nn[m]) * pl;
         fp[4] = UL * (ggm1 * pl + T(0.5) * dl * (ul * ul + vl * vl + wl * wl));
-    } else if (fabs(ML) < T(1)) {
+    } else if (abs_below_one<T>(ML)) {
         const T Mp = T(0.25) * (T(1) + ML) * (T(1) + ML);
         const T t0 = dl * cL * Mp;
         fp[0] = t0;
@@ -93,7 +116,7 @@ __device__ __forceinline__ void vanleer_g(T smallp, T gamma, T rg, T rg21, T ggm
         fp[4] = t0 * (((gamma - 1) * UL + 2 * cL) * ((gamma - 1) * UL + 2 * cL) * rg21 +
                       (ul * ul + vl * vl + wl * wl - UL * UL) * T(0.5));
     }
-    if (fabs(MR) < T(1)) {
+    if (abs_below_one<T>(MR)) {
         const T Mm = T(-0.25) * (MR - T(1)) * (MR - T(1));
         const T t0 = dr * cR * Mm;
         fm[0] = t0;
@@ -101,7 +124,7 @@ __device__ __forceinline__ void vanleer_g(T smallp, T gamma, T rg, T rg21, T ggm
         for (int m = 0; m < 3; ++m) fm[1 + m] = t0 * (nn[m] ? (-UR - T(2) * cR) * rg + rv[m] : rv[m]);
         fm[4] = t0 * (((gamma - 1) * UR - 2 * cR) * ((gamma - 1) * UR - 2 * cR) * rg21 +
                       (ur * ur + vr * vr + wr * wr - UR * UR) * T(0.5));
-    } else if (MR <= T(-1)) {
+    } else if (at_least_one<T>(-MR)) {
         fm[0] = dr * UR;
 #pragma unroll
         for (int m = 0; m < 3; ++m) fm[1 + m] = dr * UR * rv[m] + T(nn[m]) * pr;
