@@ -240,7 +240,7 @@ static ocfd_status eb_box_launch(const char* who, ocfd_context* ctx, const ocfd_
     B.visc = (flags & OCFD_VISC) != 0;
     B.redist = (flags & OCFD_REDISTRIBUTE) != 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int T = 256, sms = ctx->num_sms;
+    const int T = 128, sms = ctx->num_sms;
     k_eb_prims<<<blocks_for(plan.gcells, T, sms), T, 0, st>>>(B, ctx->parm);
     const long long fmax = std::max(plan.fcells[0], std::max(plan.fcells[1], plan.fcells[2]));
     k_eb_faces<<<dim3((unsigned)blocks_for(fmax, T, sms), 3), T, 0, st>>>(B, ctx->parm);

@@ -63,25 +63,34 @@ static double tile_work(const TileShape& s, bool visc, bool f32) {
     return w;
 }
 
-// Time of a tile shape over a set of boxes on `sms` SMs.  The pipe that
-// bounds a tile is shared by the CTAs of an SM, so a launch of n tiles takes
-// ceil(n / sms) tiles' work: large tiles have the least halo work per cell, small
-// ones spread a small box over more SMs and leave a shorter last wave.  FP64 tiles of
-// which an SM holds two keep its FP64 pipe busier (one's barriers are the other's
-// work: 8x8x4 has 12 % more work per cell than 8^3 and takes as long on large boxes,
-// 11 % less time on a slab of 512x64x4 cells than 16x8x4), hence the factor.  Measured: a
-// viscous FP64 box of 20x12x8 cells as six 8^3 tiles 207 us, as 60 tiles of 4x4x2
-// (then bound by the latency of three warps) 47 us; one of 13x97x5 cells 275 us
-// (with FP64 weights) and 44 us.  FP32 boxes take the pencil tiles: TMA staging of
-// the same shape is slower (a box of 128x96x64 cells 183 us staged, 158 us not; two
+// Time of a tile shape over a set of boxes on `sms` SMs.  The pipe that bounds a tile
+// is shared by the CTAs of an SM: large tiles have the least halo work per cell,
+// small ones spread a small box over more SMs and leave a shorter last wave.
+//   FP64  one tile's work while every tile has an SM of its own; else the cells' share
+//         of an SM (tiles that overhang the box skip what lies outside) and half a
+//         tile's work for the last wave.  Tiles of which an SM holds two keep its
+//         FP64 pipe busier (one's barriers are the other's work), hence the factor.
+//   FP32  three and more tiles share an SM and overhanging ones do all their work.
+// Measured (us, the best shape of nine unless said; the rule takes these or is within
+// 3 %): FP64 viscous box of 20x12x8 cells 49 in 60 tiles of 4x4x2, 190 in six 8^3;
+// 13x97x5 57 and 175; 32^3 127 in 8x8x4, 192 in 8^3; 61x45x37 339 in 8x8x4, 371 in
+// 8^3, 385 in 16x8x2; inviscid 128x96x64 1422 in 8^3, 1427 in 8x8x4, 1898 in 8x4x4.
+// FP32 viscous 32^3 16 in 4x4x4, 22 in 8x8x4, 27 in 8^3; inviscid 128x96x64 128 in
+// 8^3, 133 in 8x8x4.  FP32 boxes take the pencil tiles: TMA staging of the same shape
+// is slower (a box of 128x96x64 cells with face fluxes 183 us staged, 158 us not; two
 // CTAs per SM against three).
 static double tile_cost(int t, const int (*n)[3], int nbox, bool visc, bool f32, int sms) {
     const TileShape& s = kRegularTiles[t];
     long long tiles = 0;
-    for (int b = 0; b < nbox; ++b)
+    double cells = 0;
+    for (int b = 0; b < nbox; ++b) {
         tiles += (long long)((n[b][0] + s.x - 1) / s.x) * ((n[b][1] + s.y - 1) / s.y) * ((n[b][2] + s.z - 1) / s.z);
-    const double waves = tiles <= 4LL * sms ? (double)((tiles + sms - 1) / sms) : (double)tiles / sms + 0.5;
-    return waves * tile_work(s, visc, f32) * (!f32 && regular_tile_pairs(t, visc) ? 0.91 : 1.0);
+        cells += (double)n[b][0] * n[b][1] * n[b][2];
+    }
+    const double work = tile_work(s, visc, f32);
+    if (f32) return work * ((double)tiles / sms + 0.35);
+    if (tiles <= sms) return work;
+    return work * (cells / ((double)s.x * s.y * s.z * sms) + 0.5) * (regular_tile_pairs(t, visc) ? 0.91 : 1.0);
 }
 
 int pick_regular_tile(const int n[3], bool visc, bool f32, int sms) {
