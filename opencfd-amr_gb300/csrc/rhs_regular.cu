@@ -72,8 +72,8 @@ static double tile_work(const TileShape& s, bool visc, bool f32) {
 //         FP64 pipe busier (one's barriers are the other's work), hence the factor.
 //   FP32  three and more tiles share an SM and overhanging ones do all their work.
 // Measured (us, the best shape of nine unless said; the rule takes these or is within
-// 3 %): FP64 viscous box of 20x12x8 cells 49 in 60 tiles of 4x4x2, 190 in six 8^3;
-// 13x97x5 57 and 175; 32^3 127 in 8x8x4, 192 in 8^3; 61x45x37 339 in 8x8x4, 371 in
+// 3 %): FP64 viscous box of 20x12x8 cells 37 in 60 tiles of 4x4x2, 190 in six 8^3;
+// 13x97x5 58 in 4x4x4, 175 in 8^3; 32^3 127 in 8x8x4, 192 in 8^3; 61x45x37 339 in 8x8x4, 371 in
 // 8^3, 385 in 16x8x2; inviscid 128x96x64 1422 in 8^3, 1427 in 8x8x4, 1898 in 8x4x4.
 // FP32 viscous 32^3 16 in 4x4x4, 22 in 8x8x4, 27 in 8^3; inviscid 128x96x64 128 in
 // 8^3, 133 in 8x8x4.  FP32 boxes take the pencil tiles: TMA staging of the same shape

@@ -65,13 +65,21 @@ struct Pencil {
     static constexpr int FST = D == 0 ? 1 : (D == 1 ? FX : FX * FY);  // face stride along D
 };
 
+// Small FP64 tiles, of which a box has too few to fill the SMs, are bound by the
+// latency of a thread's chain of faces, not by the FP64 pipe: their WENO-Z work item
+// is one side of one face, not both sides of a run of three (a viscous box of 20x12x8
+// cells in 60 tiles of 4x4x2: 47 us in runs, 35 us this way)
+template <int TX, int TY, int TZ>
+__host__ __device__ constexpr bool tile_wide() {
+    return TX * TY * TZ <= 64;
+}
 // threads of a tile's CTA: one per cell, and in small tiles enough for the WENO-Z
 // work items of a sweep (5 components x lines x runs of three faces)
 template <int TX, int TY, int TZ>
 __host__ __device__ constexpr int tile_threads() {
     constexpr int ix = 5 * TY * TZ * ((TX + 3) / 3), iy = 5 * TX * TZ * ((TY + 3) / 3), iz = 5 * TX * TY * ((TZ + 3) / 3);
     constexpr int items = ix > iy ? (ix > iz ? ix : iz) : (iy > iz ? iy : iz), cells = TX * TY * TZ;
-    return cells >= 256 ? cells : ((items > cells ? items : cells) + 31) / 32 * 32;
+    return tile_wide<TX, TY, TZ>() ? 256 : (cells >= 256 ? cells : ((items > cells ? items : cells) + 31) / 32 * 32);
 }
 
 template <int TX, int TY, int TZ>
@@ -91,7 +99,7 @@ __host__ __device__ constexpr int face_offset() {
 template <int TX, int TY, int TZ>
 __host__ __device__ constexpr int pencil_elems() {
     return face_offset<TX, TY, TZ>() +
-           5 * max3(Pencil<0, TX, TY, TZ>::NF, Pencil<1, TX, TY, TZ>::NF, Pencil<2, TX, TY, TZ>::NF);
+           (tile_wide<TX, TY, TZ>() ? 2 : 1) * 5 * max3(Pencil<0, TX, TY, TZ>::NF, Pencil<1, TX, TY, TZ>::NF, Pencil<2, TX, TY, TZ>::NF);
 }
 
 // tiles whose cross is staged by TMA (see the file comment): the staged
@@ -487,7 +495,21 @@ __device__ __forceinline__ void sweep(const RegBoxArgs& B, const DevParm& P, int
     }
     __syncthreads();
     // ---- 2. WENO-Z face fluxes
-    if constexpr (std::is_same<FT, double>::value) {
+    if constexpr (std::is_same<FT, double>::value && tile_wide<TX, TY, TZ>()) {
+        // FP64, small tiles: a work item is one side of a face (component n), the sides
+        // in two planes, then summed; the values of the runs below
+        double* F2 = FF + 5 * max3(Pencil<0, TX, TY, TZ>::NF, Pencil<1, TX, TY, TZ>::NF, Pencil<2, TX, TY, TZ>::NF);
+        for (int it = tid; it < 10 * PC::NF; it += NT) {
+            const int n = it / PC::NF, f = it - n * PC::NF;  // n = 0..4: f+, 5..9: f-
+            const int fx = f % PC::FX, fy = (f / PC::FX) % PC::FY, fz = f / (PC::FX * PC::FY);
+            if (over && (i0 + fx > B.hi[0] + (D == 0) || j0 + fy > B.hi[1] + (D == 1) || k0 + fz > B.hi[2] + (D == 2))) continue;
+            const double* a = F + n * PC::N + fx + fy * PC::PX + fz * PC::PX * PC::PY + (n < 5 ? 0 : 5 * PC::PST);
+            const int st = n < 5 ? PC::PST : -PC::PST;
+            (n < 5 ? FF + n * PC::NF : F2 + (n - 5) * PC::NF)[f] = wenoz_1rcp(a[0], a[st], a[2 * st], a[3 * st], a[4 * st]);
+        }
+        __syncthreads();
+        for (int e = tid; e < 5 * PC::NF; e += NT) FF[e] = __dadd_rn(FF[e], F2[e]);
+    } else if constexpr (std::is_same<FT, double>::value) {
         // FP64: a work item is a run of three consecutive faces of a line along
         // D (component n); runs start every three faces, the last one at FD - 3
         // so that every stencil stays in the pencil, and a run writes only the
