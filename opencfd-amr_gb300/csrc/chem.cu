@@ -126,7 +126,7 @@ ocfd_status mech_upload(const ocfd_parm& p) {
 // mz, E (E updated), r = the 9 partial densities (updated).
 __device__ __forceinline__ void chem_cell(const double* u, double& E, double* r, double dt, const DevParm& P) {
     const double rho = dmax(u[0], P.smallr);
-    const double rhoinv = rcp_nr(rho);
+    const double rhoinv = rcp_cubic(rho);
     const double ux = u[1] * rhoinv, uy = u[2] * rhoinv, uz = u[3] * rhoinv;
     const double ei = fma(-0.5, fma(u[3], uz, fma(u[2], uy, u[1] * ux)), E);
     double cc[NSP], drho[NRE];
@@ -688,7 +688,7 @@ namespace ocfd {
 // c2prim_rgas, Source/kernel/Kernels.H:42-81
 __device__ __forceinline__ void c2prim_real(const DevParm& P, const double* u, const double* rhoi, double* q) {
     const double rho = dmax(u[0], P.smallr);
-    const double rhoinv = 1.0 / rho;
+    const double rhoinv = rcp_cubic(rho);
     const double ux = u[1] * rhoinv, uy = u[2] * rhoinv, uz = u[3] * rhoinv;
     const double kineng = 0.5 * (ux * ux + uy * uy + uz * uz);
     const double ei = u[4] - rho * kineng;
@@ -700,9 +700,9 @@ __device__ __forceinline__ void c2prim_real(const DevParm& P, const double* u, c
     const double p = ckpy(rhoi, T, P.Ru);
     q[QT] = T;
     q[QPRES] = p;
-    const double gama = p / ei + 1.0;
+    const double gama = fma(p, rcp_cubic(ei), 1.0);
     q[QGAMA] = gama;
-    q[QC] = sqrt(gama * p / rho);
+    q[QC] = sqrt(gama * p * rhoinv);
 }
 
 __global__ void __launch_bounds__(128, 4) k_chem_prims(ChemBoxArgs B, DevParm P) {
@@ -771,7 +771,7 @@ __device__ __forceinline__ void diffusion_face(const ChemBoxArgs& B, int D, int 
                                                double& muf, double& lamf, double& hflux) {
     const int li = i - (D == 0), lj = j - (D == 1), lk = k - (D == 2);
     const double rhor = B.q(i, j, k, QRHO), rhol = B.q(li, lj, lk, QRHO);
-    const double ir = rcp_nr(rhor), il = rcp_nr(rhol);
+    const double ir = rcp_cubic(rhor), il = rcp_cubic(rhol);
     const double w = 0.25 * (rhol + rhor) * B.dxinv[D];
     const double T = 0.5 * (B.q(i, j, k, QT) + B.q(li, lj, lk, QT));
     const int h = T < 1000 ? 0 : 1;
@@ -853,7 +853,7 @@ template <int D>
 __device__ __forceinline__ void chem_split(const ChemBoxArgs& B, int i, int j, int k, double* fp, double* fm) {
     const double u = B.q(i, j, k, QU), v = B.q(i, j, k, QV), w = B.q(i, j, k, QW), c = B.q(i, j, k, QC);
     const double gm1 = B.q(i, j, k, QGAMA) - 1.0;
-    const double t1 = rcp_nr(fma(2.0, gm1, 2.0)), t2 = 2.0 * gm1, t3 = (2.0 - gm1) * rcp_nr(t2);
+    const double t1 = rcp_cubic(fma(2.0, gm1, 2.0)), t2 = 2.0 * gm1, t3 = (2.0 - gm1) * rcp_cubic(t2);
     double p5[5], m5[5];
     sw_split_d<D>(B.q(i, j, k, QRHO), u, v, w, c, t1, t2, t3, gm1, p5, m5);
 #pragma unroll

@@ -161,7 +161,7 @@ __device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, d
     if (ein < emin) return tmin - (emin - ein) / ckcvbs(tmin, rhoi, Ru);
     if (ein > emax) return tmax - (emax - ein) / ckcvbs(tmax, rhoi, Ru);
     const double es = ein * c_mder.inv_ru;  // e / Ru
-    double t1 = es * rcp_nr(As);
+    double t1 = es * rcp_cubic(As);
     if (t1 < tmin || t1 > tmax) t1 = tmin + (tmax - tmin) / (emax - emin) * (ein - emin);
     const long long mag = 0x7fffffffffffffffLL;
     const double t0 = t1;
@@ -186,7 +186,7 @@ __device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, d
             d = fma(d, t1, b);
         }
         b = fma(b, t1, C[5]);
-        double dt = (es - b) * rcp_nr(d);
+        double dt = (es - b) * rcp_cubic(d);
         const long long m = __double_as_longlong(dt) & mag;
         if (m > 0x4059000000000000LL) {  // |dt| > 100 (or NaN)
             if (dt > 100.0) dt = 100.0;
@@ -373,7 +373,7 @@ __device__ __forceinline__ void eliminate(double (&U)[NRE][NRE + 1], double (&ip
             U[i][j] = sw ? t : U[i][j];
         }
     }
-    ip[C] = rcp_nr(U[C][C]);
+    ip[C] = rcp_cubic(U[C][C]);
 #pragma unroll
     for (int i = C + 1; i < NRE; ++i) {
         const double m = U[i][C] * ip[C];
@@ -392,7 +392,7 @@ __device__ __forceinline__ void chem_increment(const double* sc, double mixture,
 #pragma unroll
         for (int b = 0; b <= NRE; ++b) U[a][b] = a == b ? 1.0 : 0.0;
     const double lnT = log(T);
-    const double invT = rcp_nr(T);
+    const double invT = rcp_cubic(T);
     const double RsT = c_mder.rs * T;
     const double iRsT = c_mder.inv_rs * invT;
     double iE[NRE], z[NRE], inv[NRE];
@@ -400,7 +400,7 @@ __device__ __forceinline__ void chem_increment(const double* sc, double mixture,
         const int h = T < 1000 ? 0 : 1;
 #pragma unroll
         for (int n = 0; n < NRE; ++n) {
-            inv[n] = rcp_nr(sc[n] + 1e-20) * (dt * c_mder.inv_mw[n]);
+            inv[n] = rcp_cubic(sc[n] + 1e-20) * (dt * c_mder.inv_mw[n]);
             if (n < 2) {  // the elements: E = 1
                 iE[n] = 1.0;
                 z[n] = sc[n];
@@ -409,7 +409,7 @@ __device__ __forceinline__ void chem_increment(const double* sc, double mixture,
             const double* g = c_mder.gp[h][n - 2];
             const double t = fma(T, fma(T, fma(T, fma(T, g[4], g[3]), g[2]), g[1]), g[0]);
             const double ex = exp_tab(fma(g[5], invT, fma(g[6], lnT, t)));
-            iE[n] = rcp_nr(ex);
+            iE[n] = rcp_cubic(ex);
             z[n] = sc[n] * ex;
         }
     }
@@ -452,9 +452,9 @@ __device__ __forceinline__ void chem_increment(const double* sc, double mixture,
         const double troe_c = -0.4 - 0.67 * logFcent;
         const double troe_n = 0.75 - 1.27 * logFcent;
         const double xp = troe_c + logPred;
-        const double troe = xp * rcp_nr(fma(-0.14, xp, troe_n));
-        const double F = exp_tab(2.302585092994046 * logFcent * rcp_nr(fma(troe, troe, 1.0)));
-        return khi * (redP * rcp_nr(1.0 + redP)) * F;
+        const double troe = xp * rcp_cubic(fma(-0.14, xp, troe_n));
+        const double F = exp_tab(2.302585092994046 * logFcent * rcp_cubic(fma(troe, troe, 1.0)));
+        return khi * (redP * rcp_cubic(1.0 + redP)) * F;
     };
     const double log10e = 0.43429448190325182765;
     // 8: H + O2 (+M) <=> HO2 (+M), Fcent = 0.8
@@ -542,7 +542,7 @@ __device__ __forceinline__ void transport(double T, double p, double rho, const 
         X[n] = r[n] * c_mder.inv_mw[n];
         yow += X[n];
     }
-    const double iyow = rcp_nr(yow);
+    const double iyow = rcp_cubic(yow);
 #pragma unroll
     for (int n = 0; n < NSP; ++n) X[n] *= iyow;
     const double sqT = sqrt(T), logT = log(T), sqsqT = sqrt(sqT);
@@ -550,12 +550,12 @@ __device__ __forceinline__ void transport(double T, double p, double rho, const 
 #pragma unroll
     for (int k = 0; k < NSP; ++k) {
         sq[k] = sqsqT * poly5(logT, &c_mech.visc[k * 5]);
-        isq[k] = rcp_nr(sq[k]);
+        isq[k] = rcp_cubic(sq[k]);
         const double lam = poly5(logT, &c_mech.cond[k * 5]);  // over sqrt(T)
         s1 = fma(X[k], lam, s1);
-        s2 = fma(X[k], rcp_nr(lam), s2);
+        s2 = fma(X[k], rcp_cubic(lam), s2);
     }
-    lambda = 0.5 * sqT * (s1 + rcp_nr(s2));
+    lambda = 0.5 * sqT * (s1 + rcp_cubic(s2));
     // sum_j X_j phi_kj and sum_nn X_nn / D_(n nn), sum_nn X_nn W_nn / D_(n nn) of every
     // species (D over T^1.5)
     double ph[NSP], a1[NSP], a2[NSP], XW[NSP], W = 0.0;
@@ -576,7 +576,7 @@ __device__ __forceinline__ void transport(double T, double p, double rho, const 
             ph[k] = fma(X[j], t, ph[k]);
             ph[j] = fma(X[k], t * (v * v) * c_mder.wkj[k][j], ph[j]);  // phi_jk = phi_kj (mu_j / mu_k) (W_k / W_j)
             const int ic = j * NSP - (j * (j - 1)) / 2 + (k - j);     // upper-triangle index
-            const double ib = rcp_nr(poly5(logT, &c_mech.diff[ic * 5]));
+            const double ib = rcp_cubic(poly5(logT, &c_mech.diff[ic * 5]));
             a1[k] = fma(X[j], ib, a1[k]);
             a1[j] = fma(X[k], ib, a1[j]);
             a2[k] = fma(XW[j], ib, a2[k]);
@@ -584,11 +584,11 @@ __device__ __forceinline__ void transport(double T, double p, double rho, const 
         }
     double m = 0.0;
 #pragma unroll
-    for (int k = 0; k < NSP; ++k) m = fma(X[k] * (sq[k] * sq[k]), rcp_nr(ph[k]), m);
+    for (int k = 0; k < NSP; ++k) m = fma(X[k] * (sq[k] * sq[k]), rcp_cubic(ph[k]), m);
     mu = m;
-    const double pt = T * sqT * rcp_nr(p);
+    const double pt = T * sqT * rcp_cubic(p);
 #pragma unroll
-    for (int n = 0; n < NSP; ++n) D[n] = pt * rcp_nr(fma(a2[n], X[n] * rcp_nr(W - XW[n]), a1[n]));
+    for (int n = 0; n < NSP; ++n) D[n] = pt * rcp_cubic(fma(a2[n], X[n] * rcp_cubic(W - XW[n]), a1[n]));
 }
 
 // ---- FP32 transport of the mixed form: the same fits and mixing rules with the

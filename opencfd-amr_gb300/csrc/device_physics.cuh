@@ -134,6 +134,16 @@ __device__ __forceinline__ double rcp_nr(double x) {
     return fma(r, e, r);
 }
 
+// The same by one cubic step r (1 + e + e^2) from the seed (relative error e, so e^3
+// is below the last bit): three FMAs.  For the chemistry and transport kernels, whose
+// FP64 pipe is busy with reciprocals; the flow's primitives keep rcp_nr's last bits.
+__device__ __forceinline__ double rcp_cubic(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // WENO-Z of one split flux (Source/kernel/Reconstruction.H:83-138) in the fewest
 // FP64 operations (GB300 issues two FP64 instructions per cycle per SM).  The
 // stencil V1..V5 is ordered towards the face (f+: cells i-3..i+1; f-: cells
