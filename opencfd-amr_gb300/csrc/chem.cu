@@ -853,17 +853,22 @@ template <int D>
 __device__ __forceinline__ void chem_split(const ChemBoxArgs& B, int i, int j, int k, double* fp, double* fm) {
     const double u = B.q(i, j, k, QU), v = B.q(i, j, k, QV), w = B.q(i, j, k, QW), c = B.q(i, j, k, QC);
     const double gm1 = B.q(i, j, k, QGAMA) - 1.0;
-    const double t1 = rcp_cubic(fma(2.0, gm1, 2.0)), t2 = 2.0 * gm1, t3 = (2.0 - gm1) * rcp_cubic(t2);
+    const double t1 = rcp_cubic(fma(2.0, gm1, 2.0)), t2 = 2.0 * gm1, hc = rcp_cubic(gm1);
     double p5[5], m5[5];
-    sw_split_d<D>(B.q(i, j, k, QRHO), u, v, w, c, t1, t2, t3, gm1, p5, m5);
+    sw_split_d<D>(B.q(i, j, k, QRHO), u, v, w, c, t1, t2, hc, gm1, p5, m5);
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
         fp[n * CF_PLANE] = p5[n];
         fm[n * CF_PLANE] = m5[n];
     }
-    const double E1 = D == 0 ? u : (D == 1 ? v : w), E2 = E1 - c, E3 = E1 + c;
-    const double tp = t1 * (fma(t2, pos_part(E1), pos_part(E2)) + pos_part(E3));
-    const double tm = t1 * (fma(t2, neg_part(E1), neg_part(E2)) + neg_part(E3));
+    const double un = D == 0 ? u : (D == 1 ? v : w);
+    const SplitSide e = split_side(un, c);
+    double tB = t1 * fma(t2, un, e.outer), tS = t1 * e.inner;
+    if (e.sup) {
+        tB += tS;
+        tS = 0.0;
+    }
+    const double tp = e.up ? tB : tS, tm = e.up ? tS : tB;
 #pragma unroll
     for (int n = 0; n < NSP; ++n) {
         const double r = B.sp(i, j, k, n);

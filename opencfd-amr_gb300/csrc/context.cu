@@ -77,6 +77,7 @@ DevParm make_dev_parm(const ocfd_parm& p) {
     d.sw_tmp2 = 2.0 * (g - 1.0);
     d.sw_tmp3 = (3.0 - g) / (2.0 * (g - 1.0));
     d.sw_gm1 = g - 1;
+    d.sw_hc = 1.0 / (g - 1.0);
     d.invRg = 1.0 / d.Rg;
     d.vl_rg = 1.0 / d.gamma;
     d.vl_rg21 = 1.0 / (2.0 * (d.gamma * d.gamma - 1.0));

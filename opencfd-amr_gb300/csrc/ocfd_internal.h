@@ -18,6 +18,7 @@ struct DevParm {
     double Ru, Patm;
     double sw_tmp1, sw_tmp2, sw_tmp3;  // 1/(2g), 2(g-1), (3-g)/(2(g-1)): FluxSplit.H:31-34
     double sw_gm1;                     // (g - 1) as written `(gamma - 1)` in FluxSplit.H:41
+    double sw_hc;                      // 1/(g-1): the enthalpy's c^2 / (g - 1) of the fused FP64 split
     double invRg;                      // 1 / Rg
     double vl_rg, vl_rg21, vl_ggm1;    // 1/g, 1/(2(g^2-1)), g/(g-1): the Van Leer flux (EBkernels.H:73-171)
     double grav;                       // 0, or g = -9.8 when a call asks for OCFD_GRAVITY
