@@ -953,7 +953,7 @@ __device__ __forceinline__ void chem_face_tile(const ChemBoxArgs& B, const DevPa
 #pragma unroll 1
             for (int side = 0; side < 2; ++side) {
                 double o0, o1, o2;
-                wenoz_run3(side == 0 ? Fp + base : Fm + base + 7, side == 0 ? 1 : -1, o0, o1, o2);
+                wenoz_run3<false>(side == 0 ? Fp + base : Fm + base + 7, side == 0 ? 1 : -1, o0, o1, o2);
                 if (side == 0) {
                     p0 = o0;
                     p1 = o1;

@@ -188,9 +188,31 @@ __device__ __forceinline__ double wenoz_1rcp(double V1, double V2, double V3, do
 // run is a = f+ at the first face's stencil start, s = the pencil stride; its f-
 // side is a = f- at (start + 7 s), s = -stride, and yields the faces in reverse
 // order.
+// FLAT: look for a flat line first - the f- of a supersonic stream, an undisturbed
+// state - which has its own value at every face, all its differences being exact
+// zeros.  For the inviscid kernels, whose shocks run into undisturbed gas: a step of
+// the jet on three levels 59.5 -> 56.9 ms, the tube 2.40 -> 2.34 ms, the blast 5.67 ->
+// 5.60 ms; states without such lines lose 0.2 % to the test (the viscous box) to 0.5 %
+// (the multispecies box), so those kernels go without.
+template <bool FLAT>
 __device__ __forceinline__ void wenoz_run3(const double* a, int s, double& o0, double& o1, double& o2) {
     double V3 = a[2 * s], V4 = a[3 * s], V5 = a[4 * s];
     const double V1 = a[0], V2 = a[s];
+    if constexpr (FLAT) {
+        // the high words of two cells send nearly every other line on
+        const auto hi = [](double v) { return (unsigned)__double2hiint(v); };
+        const auto lo = [](double v) { return (unsigned)__double2loint(v); };
+        const unsigned h = hi(V1), l = lo(V1);
+        if (hi(V5) == h) {
+            const double V6 = a[5 * s], V7 = a[6 * s];
+            const unsigned off = (hi(V2) ^ h) | (lo(V2) ^ l) | (hi(V3) ^ h) | (lo(V3) ^ l) | (hi(V4) ^ h) |
+                                 (lo(V4) ^ l) | (lo(V5) ^ l) | (hi(V6) ^ h) | (lo(V6) ^ l) | (hi(V7) ^ h) | (lo(V7) ^ l);
+            if (off == 0u && (h & 0x7ff00000u) != 0x7ff00000u) {
+                o0 = o1 = o2 = V1;
+                return;
+            }
+        }
+    }
     const double d1 = __dsub_rn(V2, V1);
     double d2 = __dsub_rn(V3, V2), d3 = __dsub_rn(V4, V3), d4 = __dsub_rn(V5, V4);
     double e1 = __dsub_rn(d2, d1), e2 = __dsub_rn(d3, d2), e3 = __dsub_rn(d4, d3);

@@ -543,7 +543,7 @@ __device__ __forceinline__ void sweep(const RegBoxArgs& B, const DevParm& P, int
                 const double* a = side == 0 ? F + n * PC::N + base : F + (5 + n) * PC::N + base + 7 * PC::PST;
                 const int st = side == 0 ? PC::PST : -PC::PST;
                 double o0, o1, o2;
-                wenoz_run3(a, st, o0, o1, o2);
+                wenoz_run3<!VISC>(a, st, o0, o1, o2);
                 if (side == 0) {
                     p0 = o0;
                     p1 = o1;
