@@ -163,19 +163,17 @@ __device__ __forceinline__ double rcp_cubic(double x) {
 //     differences only.
 // The same value up to rounding (parity tests: 1e-12 per right-hand side), finite
 // for flux differences below ~1e150.  Differences and curvature terms belong to
-// cells of the line and serve neighbouring faces: 13 FP64 operations per face and
-// side in runs of three faces (17 for a face alone).  With indicators and candidates
+// cells of the line and serve neighbouring faces: 10 FP64 operations per face and
+// side in runs of three faces (13 for a face alone).  With indicators and candidates
 // formed from the values and all of it in FP64 they were 49 (54), and a stage of the
-// 3D blast on 128x128x64 cells took 4.00 ms; this way 1.91 ms (1.79 ms with the
-// split of split_side below).
+// 3D blast on 128x128x64 cells took 4.00 ms; this way and with the split of split_side
+// below, 1.73 ms.
 // Every rounding is written out, so the value does not depend on the code around
 // the call.
 __device__ __forceinline__ double wenoz_face_d(double V3, double d2, double d3, double e1, double e2, double e3,
                                                const wz::Num& k1, const wz::Num& k2, const wz::Num& k3) {
     const double g1 = __fma_rn(2.0, d2, e1), g2 = __dadd_rn(d2, d3), g3 = __fma_rn(2.0, d3, -e3);
-    double c1, c2, c3;
-    wz::weights(g1, g2, g3, k1, k2, k3, c1, c2, c3);
-    const double corr = __fma_rn(c3, __fma_rn(3.0, e2, -e3), __fma_rn(c2, e2, __dmul_rn(c1, e1)));
+    const double corr = wz::correction(wz::weights(g1, g2, g3, k1, k2, k3), e1, e2, __fma_rn(3.0, e2, -e3));
     return __dadd_rn(__fma_rn(0.5, d2, V3), corr);
 }
 __device__ __forceinline__ double wenoz_1rcp(double V1, double V2, double V3, double V4, double V5) {

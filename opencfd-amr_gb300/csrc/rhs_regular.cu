@@ -30,7 +30,7 @@ static bool regular_tile_pairs(int tile, bool visc) {
 }
 
 const TileShape kRegularTiles[] = {{8, 8, 8, 0},  {8, 8, 4, 0}, {16, 8, 4, 0}, {16, 16, 2, 0}, {32, 8, 2, 0},
-                                   {16, 8, 2, 0}, {8, 8, 8, 1}, {8, 8, 4, 1}, {16, 8, 4, 1}, {8, 4, 4, 0}, {4, 4, 4, 0},  {4, 4, 2, 0}};
+                                   {16, 8, 2, 0}, {8, 8, 8, 1}, {8, 8, 4, 1}, {16, 8, 4, 1}, {8, 4, 4, 0}, {4, 4, 4, 0},  {4, 4, 2, 0}, {8, 2, 2, 0}};
 const int kNumRegularTiles = sizeof(kRegularTiles) / sizeof(kRegularTiles[0]);
 const int kNumPublicTiles = 9;
 
@@ -72,9 +72,11 @@ static double tile_work(const TileShape& s, bool visc, bool f32) {
 //         FP64 pipe busier (one's barriers are the other's work), hence the factor.
 //   FP32  three and more tiles share an SM and overhanging ones do all their work.
 // Measured (us, the best shape of nine unless said; the rule takes these or is within
-// 3 %): FP64 viscous box of 20x12x8 cells 37 in 60 tiles of 4x4x2, 190 in six 8^3;
-// 13x97x5 58 in 4x4x4, 175 in 8^3; 32^3 127 in 8x8x4, 192 in 8^3; 61x45x37 339 in 8x8x4, 371 in
-// 8^3, 385 in 16x8x2; inviscid 128x96x64 1422 in 8^3, 1427 in 8x8x4, 1898 in 8x4x4.
+// 3 %): FP64 viscous box of 20x12x8 cells 33 in 60 tiles of 4x4x2, 190 in six 8^3;
+// 13x97x5 45 in 8x2x2, 52 in 4x4x4; with the arithmetic before the split's and the
+// correction's last regrouping (1.1 times these) 175 in 8^3, 32^3 127 in 8x8x4, 192 in
+// 8^3, 61x45x37 339 in 8x8x4, 371 in 8^3, inviscid 128x96x64 1422 in 8^3, 1427 in
+// 8x8x4, 1898 in 8x4x4.
 // FP32 viscous 32^3 16 in 4x4x4, 22 in 8x8x4, 27 in 8^3; inviscid 128x96x64 128 in
 // 8^3, 133 in 8x8x4.  FP32 boxes take the pencil tiles: TMA staging of the same shape
 // is slower (a box of 128x96x64 cells with face fluxes 183 us staged, 158 us not; two
@@ -89,7 +91,9 @@ static double tile_cost(int t, const int (*n)[3], int nbox, bool visc, bool f32,
     }
     const double work = tile_work(s, visc, f32);
     if (f32) return work * ((double)tiles / sms + 0.35);
-    if (tiles <= sms) return work;
+    if (tiles <= sms) return t == 12 ? 1.05 * work : work;  // 8x2x2: 256 threads (34.9 us against 32.8)
+    // an SM holds one 4x4x2 tile (480 threads), and all take alike
+    if (t == 11) return work * (double)((tiles + sms - 1) / sms);
     return work * (cells / ((double)s.x * s.y * s.z * sms) + 0.5) * (regular_tile_pairs(t, visc) ? 0.91 : 1.0);
 }
 
@@ -98,7 +102,7 @@ int pick_regular_tile(const int n[3], bool visc, bool f32, int sms) {
     int best = 1;
     double best_cost = 1e300;
     for (int t = 0; t < kNumRegularTiles; ++t) {
-        if (!regular_tile_fits(t, visc) || kRegularTiles[t].staged) continue;
+        if (!regular_tile_fits(t, visc) || kRegularTiles[t].staged || (f32 && t == 12)) continue;  // 8x2x2: FP64's
         const double cost = tile_cost(t, one, 1, visc, f32, sms);
         if (cost < best_cost * 0.999) {
             best_cost = cost;

@@ -65,21 +65,33 @@ struct Pencil {
     static constexpr int FST = D == 0 ? 1 : (D == 1 ? FX : FX * FY);  // face stride along D
 };
 
+__host__ __device__ constexpr int max3(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
 // Small FP64 tiles, of which a box has too few to fill the SMs, are bound by the
 // latency of a thread's chain of faces, not by the FP64 pipe: their WENO-Z work item
 // is one side of one face, not both sides of a run of three (a viscous box of 20x12x8
-// cells in 60 tiles of 4x4x2: 47 us in runs, 35 us this way)
+// cells in 60 tiles of 4x4x2: 47 us in runs, 35 us this way, 32.8 us with 480 threads)
 template <int TX, int TY, int TZ>
 __host__ __device__ constexpr bool tile_wide() {
     return TX * TY * TZ <= 64;
 }
 // threads of a tile's CTA: one per cell, and in small tiles enough for the WENO-Z
-// work items of a sweep (5 components x lines x runs of three faces)
-template <int TX, int TY, int TZ>
+// work items of a sweep (5 components x lines x runs of three faces).  In FP64 a 4x4x2
+// tile takes all its one-sided items at once, for boxes whose tiles have an SM each;
+// 4x4x4 in three rounds and 8x2x2 in two, so that an SM holds two and more
+// (256 threads each -> 480 and 288, with the integer correction of weno_weights.cuh:
+// viscous 20x12x8 cells in 4x4x2 34.9 -> 32.8 us, 24x20x16 in 4x4x4 45.9 -> 43.9 us;
+// inviscid 13x97x5, some 300 tiles of 32 cells: 39.8 us in 4x4x4, 31.5 in 8x2x2).
+// FP32 boxes large enough to fill the SMs lost 20 % to more than 256.
+template <class FT, int TX, int TY, int TZ>
 __host__ __device__ constexpr int tile_threads() {
     constexpr int ix = 5 * TY * TZ * ((TX + 3) / 3), iy = 5 * TX * TZ * ((TY + 3) / 3), iz = 5 * TX * TY * ((TZ + 3) / 3);
     constexpr int items = ix > iy ? (ix > iz ? ix : iz) : (iy > iz ? iy : iz), cells = TX * TY * TZ;
-    return tile_wide<TX, TY, TZ>() ? 256 : (cells >= 256 ? cells : ((items > cells ? items : cells) + 31) / 32 * 32);
+    if (tile_wide<TX, TY, TZ>()) {
+        if (!std::is_same<FT, double>::value || TY < 4) return 256;
+        constexpr int sides = 10 * max3(Pencil<0, TX, TY, TZ>::NF, Pencil<1, TX, TY, TZ>::NF, Pencil<2, TX, TY, TZ>::NF);
+        return ((sides <= 512 ? sides : (sides + 2) / 3) + 31) / 32 * 32;
+    }
+    return cells >= 256 ? cells : ((items > cells ? items : cells) + 31) / 32 * 32;
 }
 
 template <int TX, int TY, int TZ>
@@ -91,7 +103,6 @@ struct Ring {
 // The split pencils (10 values per cell) and, behind the longest of them, the face
 // fluxes (5 per face): at one place for the three sweeps, so that a sweep's cells can
 // be split while the last one's face fluxes are still read.
-__host__ __device__ constexpr int max3(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
 template <int TX, int TY, int TZ>
 __host__ __device__ constexpr int face_offset() {
     return 10 * max3(Pencil<0, TX, TY, TZ>::N, Pencil<1, TX, TY, TZ>::N, Pencil<2, TX, TY, TZ>::N);
@@ -331,7 +342,7 @@ template <int TX, int TY, int TZ>
 __device__ __forceinline__ void cross_prims(const RegBoxArgs& B, const DevParm& P, int i0, int j0, int k0,
                                             const double* stage, bool staged, float* Q) {
     using C = Cross<TX, TY, TZ>;
-    constexpr int NT = tile_threads<TX, TY, TZ>();
+    constexpr int NT = tile_threads<float, TX, TY, TZ>();
     for (int idx = threadIdx.x; idx < C::NQ; idx += NT) {
         int x, y, z, so, sc;
         bool zhalo = false;
@@ -394,7 +405,7 @@ template <int TX, int TY, int TZ>
 __device__ __forceinline__ void cross_prims_plain(const RegBoxArgs& B, const DevParm& P, int i0, int j0, int k0,
                                                   double* Q) {
     using C = Cross<TX, TY, TZ>;
-    constexpr int NT = tile_threads<TX, TY, TZ>();
+    constexpr int NT = tile_threads<double, TX, TY, TZ>();
     for (int idx = threadIdx.x; idx < C::NQ; idx += NT) {
         int x, y, z;
         if (idx < C::NC) {
@@ -438,7 +449,7 @@ template <class FT, int D, int TX, int TY, int TZ, bool VISC, bool CROSS = false
 __device__ __forceinline__ void sweep(const RegBoxArgs& B, const DevParm& P, int i0, int j0, int k0,
                                       FT* F, FT* FF, const FT* ring, FT* acc, const FT* Q = nullptr) {
     using PC = Pencil<D, TX, TY, TZ>;
-    constexpr int NT = tile_threads<TX, TY, TZ>();
+    constexpr int NT = tile_threads<FT, TX, TY, TZ>();
     const int tid = threadIdx.x;
     // an FP64 tile that overhangs the box: its faces outside are not formed (nothing
     // reads them; a box of 61x45x37 cells is a fifth padding in 8^3 tiles).  The FP32
@@ -639,7 +650,7 @@ __device__ __forceinline__ void rhs_tile(const RegBoxArgs* __restrict__ boxes, c
                                          int nbox, const RegBoxArgs& single, const DevParm& P, int t,
                                          unsigned char* sbase, uint64_t* bar, uint32_t& phase, bool& abort,
                                          double& local_dt) {
-    constexpr int NT = tile_threads<TX, TY, TZ>();
+    constexpr int NT = tile_threads<FT, TX, TY, TZ>();
     // locate the box of this tile: a single box, or a prefix table over a box list
     int b = 0;
     if (boxes) {
@@ -789,16 +800,16 @@ __device__ __forceinline__ void rhs_tile(const RegBoxArgs* __restrict__ boxes, c
 template <class FT, int TX, int TY, int TZ, bool VISC, bool XS>
 __host__ __device__ constexpr int regular_min_blocks() {
     if (std::is_same<FT, double>::value)  // the WENO-Z runs take up to 128 registers
-        return tile_threads<TX, TY, TZ>() <= 256 && 2 * (regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>() + 1024) <= 228 * 1024 ? 2 : 1;
+        return tile_threads<FT, TX, TY, TZ>() <= 288 && 2 * (regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>() + 1024) <= 228 * 1024 ? 2 : 1;
     const int b = (int)((228u * 1024u) / (regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>() + 1024u));
-    const int t = 2048 / tile_threads<TX, TY, TZ>();
+    const int t = 2048 / tile_threads<FT, TX, TY, TZ>();
     int m = b < t ? b : t;
     m = m < 3 ? m : 3;
     return m < 1 ? 1 : m;
 }
 
 template <class FT, int TX, int TY, int TZ, bool VISC, bool XS>
-__global__ void __launch_bounds__((tile_threads<TX, TY, TZ>()), (regular_min_blocks<FT, TX, TY, TZ, VISC, XS>()))
+__global__ void __launch_bounds__((tile_threads<FT, TX, TY, TZ>()), (regular_min_blocks<FT, TX, TY, TZ, VISC, XS>()))
     k_rhs_regular(const RegBoxArgs* __restrict__ boxes, const int* __restrict__ tile_start,
                   int nbox, const __grid_constant__ RegBoxArgs single, DevParm P, int ntiles, int sched,
                   unsigned* queue) {
@@ -854,7 +865,7 @@ template <class FT, int TX, int TY, int TZ, bool VISC, bool XS>
 static ocfd_status launch_t(const RegBoxArgs* d_boxes, const int* d_tile_start, int nbox,
                             const RegBoxArgs& single, int ntiles, const DevParm& P,
                             cudaStream_t st, int sched, unsigned* queue) {
-    constexpr int NT = tile_threads<TX, TY, TZ>();
+    constexpr int NT = tile_threads<FT, TX, TY, TZ>();
     constexpr size_t smem = regular_smem_bytes<FT, TX, TY, TZ, VISC, XS>();
     auto kern = k_rhs_regular<FT, TX, TY, TZ, VISC, XS>;
     if (smem > kMaxSmem) return fail(OCFD_BAD_ARG, "regular RHS tile does not fit shared memory in this mode");
@@ -894,7 +905,7 @@ static bool configure_one() {
 #define OCFD_REGULAR_TILES(X)                                                                              \
     X(0, 8, 8, 8, false) X(1, 8, 8, 4, false) X(2, 16, 8, 4, false) X(3, 16, 16, 2, false) X(4, 32, 8, 2, false) \
         X(5, 16, 8, 2, false) X(6, 8, 8, 8, true) X(7, 8, 8, 4, true) X(8, 16, 8, 4, true)                          \
-    X(9, 8, 4, 4, false) X(10, 4, 4, 4, false) X(11, 4, 4, 2, false)
+    X(9, 8, 4, 4, false) X(10, 4, 4, 4, false) X(11, 4, 4, 2, false) X(12, 8, 2, 2, false)
 
 template <class FT>
 struct StagedIn {  // the staged variants exist in the FP32-flux form only

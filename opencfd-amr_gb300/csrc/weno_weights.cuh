@@ -11,12 +11,16 @@
 // coefficients' error is 0.5e-16 rms, where the same formulas in FP64 have 0.8e-16 to
 // 6e-16; where tau cancels both lose digits, this form six bits fewer.  Exponents are
 // integers, so no intermediate overflows or underflows.
-// They replace 24 of 37 FP64 operations of a face and side by about 400 integer
+// They replace 27 of 37 FP64 operations of a face and side by about 450 integer
 // instructions, which run in the FP64 pipe's shadow.  A stage of the 3D blast on
 // 128x128x64 cells: 3.32 ms in FP64; 2.38 ms with the weights here; 2.17 ms with
 // the division too; 1.91 ms with the indicators too (808 instead of 1630 FP64
-// instructions per cell, the FP64 pipe 74 % busy, 1.26 instead of 0.37 instructions
-// issued per cycle).
+// instructions per cell).  With the split's 14 operations less 1.79 ms (750); with the
+// correction formed here too, 1.73 ms (649 per cell, the FP64 pipe 65 % busy, 1.49
+// instead of 0.37 instructions issued per cycle): the integer chain's latency on 16
+// warps per SM now weighs as much as the FP64 pipe.  128-bit arithmetic on faces of
+// smooth, random and jumping lines puts the face value's rms error at 0.95 of that of
+// FP64 coefficients (smooth, random), 1.0 (jumps).
 #pragma once
 
 #include <cstdint>
@@ -118,6 +122,7 @@ OCFD_HD uint64_t recip(uint64_t m) {
     return ((uint64_t)y << 32) + (uint64_t)(((int64_t)ch * (int64_t)y) >> 8) + (((uint64_t)cl * y) >> 30) - 8;
 }
 
+OCFD_HD bool negative(double x) { return (int64_t)bits_of(x) < 0; }
 // |x| as a square's factor: m in [2^62, 2^63), biased exponent
 OCFD_HD Num unpack_abs(double x) {
     const uint64_t b = bits_of(x) & 0x7fffffffffffffffull;
@@ -148,13 +153,17 @@ OCFD_HD Num difference(const Num& a, const Num& b) {
     return Num{m << z, x - z};
 }
 
-// The WENO-Z correction's coefficients: with D_k = 12 (eps + beta_k) from the first
-// differences g_k = 2 sqrt(beta_k - 13/12 e_k^2) and the curvature terms of the three
-// sub-stencils, tau = |D_1 - D_3|, q_k = D_k^2, A_k = q_i q_j (q_k + tau^2) ({i, j} the
-// other two) and s = A_1 + 6 A_2 + 3 A_3: c1 = A_1 / (3 s), c2 = 6 A_2 / (3 s), c3 =
-// 3 A_3 / (6 s).
-OCFD_HD void weights(double g1, double g2, double g3, const Num& k1, const Num& k2, const Num& k3, double& c1,
-                     double& c2, double& c3) {
+// The weights of the three candidates' second differences: with D_k = 12 (eps +
+// beta_k) from the first differences g_k = 2 sqrt(beta_k - 13/12 e_k^2) and the
+// curvature terms of the three sub-stencils, tau = |D_1 - D_3|, q_k = D_k^2 and
+// A_k = q_i q_j (q_k + tau^2) ({i, j} the other two), b = (A_1, 6 A_2, 3 A_3) and
+// 1 / (3 (b1 + b2 + b3)) = z 2^(-125 - e).
+struct Weights {
+    Num b1, b2, b3;
+    uint64_t z;
+    int e;
+};
+OCFD_HD Weights weights(double g1, double g2, double g3, const Num& k1, const Num& k2, const Num& k3) {
     const Num d1 = indicator(g1, k1), d2 = indicator(g2, k2), d3 = indicator(g3, k3), t = difference(d1, d3);
     const uint64_t q1 = sq_hi(d1.m), q2 = sq_hi(d2.m), q3 = sq_hi(d3.m), tt = sq_hi(t.m);  // [2^60, 2^62)
     const int e1 = 2 * d1.e, e2 = 2 * d2.e, e3 = 2 * d3.e, et = 2 * t.e;
@@ -164,16 +173,37 @@ OCFD_HD void weights(double g1, double g2, double g3, const Num& k1, const Num& 
     const uint64_t s3 = shr(q3, imax(et - e3, 0)) + shr(tt, imax(e3 - et, 0));  // [2^60, 2^63)
     const uint64_t r23 = mul_hi(2 * q2, 2 * q3) * 2, r13 = mul_hi(2 * q1, 2 * q3) * 2, r12 = mul_hi(2 * q1, 2 * q2) * 2;
     // A_k in [2^55, 2^62); the constant exponent offsets are common to all three
-    const Num b1 = normalise(mul_hi(r23, s1), e2 + e3 + imax(e1, et));
-    const Num b2 = normalise(3 * (mul_hi(r13, s2) >> 1), e1 + e3 + imax(e2, et) + 2);  // 6 A_2
-    const Num b3 = normalise(3 * (mul_hi(r12, s3) >> 1), e1 + e2 + imax(e3, et) + 1);  // 3 A_3
-    const int top = imax(b1.e, imax(b2.e, b3.e)) + 4;
-    const Num s = normalise(3 * (shr(b1.m, top - b1.e) + shr(b2.m, top - b2.e) + shr(b3.m, top - b3.e)), top);  // 3 s
-    const uint64_t z = recip(s.m);
-    // b / (3 s) = b.m z 2^-125 2^(b.e - s.e)
-    c1 = pack(normalise(mul_hi(b1.m, z), b1.e - s.e - 61));
-    c2 = pack(normalise(mul_hi(b2.m, z), b2.e - s.e - 61));
-    c3 = pack(normalise(mul_hi(b3.m, z), b3.e - s.e - 62));
+    Weights w;
+    w.b1 = normalise(mul_hi(r23, s1), e2 + e3 + imax(e1, et));
+    w.b2 = normalise(3 * (mul_hi(r13, s2) >> 1), e1 + e3 + imax(e2, et) + 2);  // 6 A_2
+    w.b3 = normalise(3 * (mul_hi(r12, s3) >> 1), e1 + e2 + imax(e3, et) + 1);  // 3 A_3
+    const int top = imax(w.b1.e, imax(w.b2.e, w.b3.e)) + 4;
+    const Num s =
+        normalise(3 * (shr(w.b1.m, top - w.b1.e) + shr(w.b2.m, top - w.b2.e) + shr(w.b3.m, top - w.b3.e)), top);  // 3 s
+    w.z = recip(s.m);
+    w.e = s.e;
+    return w;
+}
+
+// The correction (b1 e1 + b2 e2 + b3 h / 2) / (3 s), h = 3 e2 - e3, to the face value
+// V3 + d2 / 2, rounded once.  The products are aligned to the largest of them, so
+// what is cut off stays below 2^-57 of it; factors below 2^-1022 count as zero, and
+// the result is not a number if one of them is not finite.
+OCFD_HD double correction(const Weights& w, double e1, double e2, double h) {
+    const Num a1 = unpack_abs(e1), a2 = unpack_abs(e2), a3 = unpack_abs(h);
+    const int big = imax(a1.e, imax(a2.e, a3.e));
+    if (big == 0) return 0.0;
+    const int x1 = w.b1.e + a1.e, x2 = w.b2.e + a2.e, x3 = w.b3.e - 1 + a3.e;
+    const int top = imax(x1, imax(x2, x3)) + 1;
+    const int64_t p1 = (int64_t)shr(mul_hi(w.b1.m, a1.m), top - x1), p2 = (int64_t)shr(mul_hi(w.b2.m, a2.m), top - x2),
+                  p3 = (int64_t)shr(mul_hi(w.b3.m, a3.m), top - x3);  // below 2^61 each
+    const int64_t sum = (negative(e1) ? -p1 : p1) + (negative(e2) ? -p2 : p2) + (negative(h) ? -p3 : p3);
+    const uint64_t m = (uint64_t)(sum < 0 ? -sum : sum);
+    const int z = ((m >> 32) ? lead_zeros((uint32_t)(m >> 32)) : 32 + lead_zeros((uint32_t)m | 1u)) - 1;
+    // |e_k| = a.m 2^(a.e - 1085), a product's high half 2^64, z 2^-125 and its high half 2^64
+    const double c = pack(normalise(mul_hi(m << z, w.z), top - z - w.e - 1085 + 64 - 61));
+    if (m == 0 || big == 0x7ff) return big == 0x7ff ? double_of(0x7ff8000000000000ull) : 0.0;
+    return double_of(bits_of(c) | ((uint64_t)sum & 0x8000000000000000ull));
 }
 
 }  // namespace wz

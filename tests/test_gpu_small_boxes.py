@@ -1,5 +1,5 @@
 """Per-box right-hand sides of boxes that take the small tile shapes (8x4x4, 4x4x4,
-4x4x2), with remainders in every direction: bit for bit the values of the same
+4x4x2, 8x2x2), with remainders in every direction: bit for bit the values of the same
 cells and faces in a call on the whole box, which takes 8^3 tiles."""
 import pytest
 
@@ -27,7 +27,7 @@ def rhs(ctx, S, lo, hi, flags):
     return [dS] + fl
 
 
-@pytest.mark.parametrize("n", [(1, 1, 1), (4, 4, 2), (5, 3, 7), (9, 17, 2), (20, 12, 8), (31, 5, 18)])
+@pytest.mark.parametrize("n", [(1, 1, 1), (4, 4, 2), (5, 3, 7), (9, 17, 2), (20, 12, 8), (31, 5, 18), (30, 31, 5)])
 @pytest.mark.parametrize("visc", [0, 1])
 @pytest.mark.parametrize("fp32", [0, 4])
 def test_small_box_equals_whole(whole, n, visc, fp32):

@@ -19,13 +19,16 @@ def weights(tmp_path_factory):
     src, so = d / "wz.cpp", d / "wz.so"
     src.write_text('#include "weno_weights.cuh"\n'
                    'using namespace ocfd::wz;\n'
-                   'extern "C" void w(const double* g, const double* e, double* c) '
-                   '{ weights(g[0], g[1], g[2], curvature(e[0]), curvature(e[1]), curvature(e[2]), c[0], c[1], c[2]); }\n')
+                   'extern "C" void w(const double* g, const double* e, double* c) {\n'
+                   '  Weights w = weights(g[0], g[1], g[2], curvature(e[0]), curvature(e[1]), curvature(e[2]));\n'
+                   '  auto over = [&](Num b, int s) { return pack(normalise(mul_hi(b.m, w.z), b.e - w.e - 61 - s)); };\n'
+                   '  c[0] = over(w.b1, 0); c[1] = over(w.b2, 0); c[2] = over(w.b3, 1);\n'
+                   '  c[3] = correction(w, e[0], e[1], __builtin_fma(3.0, e[1], -e[2])); }\n')
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(so)], check=True)
     lib = ctypes.CDLL(str(so))
 
     def f(g, e):
-        c = (ctypes.c_double * 3)()
+        c = (ctypes.c_double * 4)()
         lib.w((ctypes.c_double * 3)(*g), (ctypes.c_double * 3)(*e), c)
         return list(c)
     return f
@@ -66,7 +69,11 @@ def test_weights_exact(weights, lo, hi):
         if n % 5 == 4:
             g[n % 3], e[(n + 1) % 3] = 0.0, 0.0
         want, amp = exact_coefficients(g, e)
-        for got, w in zip(weights(g, e), want):
+        c = weights(g, e)
+        # the correction: each coefficient's error, one rounding, the alignment's 2^-57
+        terms = [want[0] * Q(e[0]), want[1] * Q(e[1]), 3 * want[2] * Q(e[1]), -want[2] * Q(e[2])]
+        assert abs(Q(c[3]) - sum(terms)) <= (Q(TOL) + 2 * amp) * sum(abs(t) for t in terms)
+        for got, w in zip(c, want):
             if w < Q(2) ** -1000:
                 assert 0 <= got <= 2.0 ** -999
             else:
@@ -77,14 +84,23 @@ def test_weights_flat(weights):
     # zero and denormal differences: the linear weights
     for x in (0.0, 5e-324, 1e-310, 1e-200):
         c = weights([x, -x, 0.0], [x, 0.0, -x])
-        assert np.allclose(c, [1 / 30, 6 / 30, 3 / 60], rtol=2 ** -52, atol=0)
+        assert np.allclose(c[:3], [1 / 30, 6 / 30, 3 / 60], rtol=2 ** -52, atol=0)
+    assert weights([0.0] * 3, [0.0, -0.0, 0.0])[3] == 0.0 and weights([1.0, 2.0, -3.0], [0.0] * 3)[3] == 0.0
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_correction_not_finite(weights, bad):
+    for k in range(3):
+        e = [1.0, -2.0, 0.5]
+        e[k] = bad
+        assert np.isnan(weights([1.0, 1.0, bad], e)[3])
 
 
 def face(weights, V):
     d = [V[i + 1] - V[i] for i in range(4)]
     e = [d[i + 1] - d[i] for i in range(3)]
     c = weights([2 * d[1] + e[0], d[1] + d[2], 2 * d[2] - e[2]], e)
-    return (V[2] + 0.5 * d[1]) + (c[0] * e[0] + c[1] * e[1] + c[2] * (3 * e[1] - e[2]))
+    return (V[2] + 0.5 * d[1]) + c[3]
 
 
 def face_exact(V):
