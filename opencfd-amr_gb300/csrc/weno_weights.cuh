@@ -144,13 +144,16 @@ OCFD_HD Num indicator(double g, const Num& c) {
     const int x = 2 * a.e + 2;
     return normalise(shr((sq_hi(a.m) >> 2) * 3, imax(c.e - x, 0)) + shr(c.m, imax(x - c.e, 0)), imax(x, c.e));
 }
-// |a - b|, m in [2^62, 2^63) or 0
+// |a - b|, m in [2^62, 2^63), or 0 with an exponent whose double lies below every
+// indicator's, so that the square aligns nothing else away (an exponent next to a's,
+// as cancelled digits leave it, shifted the middle indicator out where the outer two
+// are equal and 2^62 times larger)
 OCFD_HD Num difference(const Num& a, const Num& b) {
     const int x = imax(a.e, b.e);
     const int64_t d = (int64_t)(shr(a.m, x - a.e) - shr(b.m, x - b.e));
     const uint64_t m = (uint64_t)(d < 0 ? -d : d);
     const int z = ((m >> 32) ? lead_zeros((uint32_t)(m >> 32)) : 32 + lead_zeros((uint32_t)m | 1u)) - 1;
-    return Num{m << z, x - z};
+    return Num{m << z, m ? x - z : x - 8192};
 }
 
 // The weights of the three candidates' second differences: with D_k = 12 (eps +

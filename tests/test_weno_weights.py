@@ -128,3 +128,20 @@ def test_face_value(weights, scale):
         # indicators within 10 roundings, which the weights double; candidates of at most
         # 7 max |V| with the weights' errors; four roundings of the sum
         assert abs(Q(face(weights, V)) - face_exact(V)) <= Q(2.0 ** -53 * 200 * max(abs(x) for x in V))
+
+
+@pytest.mark.parametrize("mid", [0.0, 1e-3, 1.0, 30.0])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("p", range(3, 16))
+def test_plateau_between_equal_jumps(weights, p, sign, mid):
+    # tau is exactly zero, the middle indicator far below the outer two: the linear
+    # weights, whatever the indicators' ratio
+    a = 10.0 ** p
+    g, e = [a, mid, sign * a], [a, 0.0, -sign * a]
+    c = weights(g, e)
+    for got, w in zip(c, (Q(1, 30), Q(1, 5), Q(1, 20))):
+        assert abs(Q(got) - w) <= Q(TOL) * w
+    V = [1.0 + a, 1.0, 1.0, 1.0, 1.0 + sign * a]
+    # the values' differences are exact; three terms of at most a / 5, each within TOL,
+    # and two roundings of the sum
+    assert abs(Q(face(weights, V)) - face_exact(V)) <= (Q(TOL) + Q(2.0 ** -52)) * Q(a)
