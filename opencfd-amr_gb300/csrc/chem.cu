@@ -55,7 +55,7 @@ ocfd_status mech_upload(const ocfd_parm& p) {
         }
     for (int a = 0; a < NSP; ++a) {
         md.inv_mw[a] = 1.0 / t.mw[a];
-        md.hw[a] = -t.HP[a] * p.Ru * md.inv_mw[a];
+        md.hpw[a] = -t.HP[a] * md.inv_mw[a];
         md.a0w[a] = t.A0[a] * md.inv_mw[a];
         for (int k = 0; k < 5; ++k) md.nw[k][a] = k * t.mw[a];
         for (int h = 0; h < 2; ++h) {
@@ -93,9 +93,6 @@ ocfd_status mech_upload(const ocfd_parm& p) {
             const double g[7] = {a[0] - a[6], -a[1] / 2.0, -a[2] / 6.0, -a[3] / 12.0, -a[4] / 20.0, a[5], -a[0]};
             for (int k = 0; k < 7; ++k) md.gp[h][n][k] = g[k];
         }
-    md.inv_ru = 1.0 / p.Ru;
-    md.rs = p.Ru / p.Patm * 1e6;
-    md.inv_rs = 1.0 / md.rs;
     if (cudaMemcpyToSymbol(c_mder, &md, sizeof(md)) != cudaSuccess) {
         cudaError_t e = cudaGetLastError();
         return fail(OCFD_LAUNCH_FAIL, std::string("mechanism upload: ") + cudaGetErrorString(e));
@@ -130,23 +127,23 @@ __device__ __forceinline__ void chem_cell(const double* u, double& E, double* r,
     const double ux = u[1] * rhoinv, uy = u[2] * rhoinv, uz = u[3] * rhoinv;
     const double ei = fma(-0.5, fma(u[3], uz, fma(u[2], uy, u[1] * ux)), E);
     double cc[NSP], drho[NRE];
-    const double T = get_t_given_ey(ei, r, P.Ru);
+    const double T = get_t_given_ey(ei, r, P);
     double mixture = 0.0;
 #pragma unroll
     for (int n = 0; n < NSP; n++) {
         cc[n] = r[n] * c_mder.inv_mw[n] * 1e-6;
         mixture += cc[n];
     }
-    chem_increment(cc, mixture, T, dt, drho);
+    chem_increment(cc, mixture, T, dt, P, drho);
     double dei = 0;
 #pragma unroll
     for (int n = 0; n < NRE; ++n) {
         const double v = r[n] + drho[n];
         r[n] = v < 0 ? 0.0 : v;
-        dei = fma(c_mder.hw[n], drho[n], dei);
+        dei = fma(c_mder.hpw[n], drho[n], dei);
     }
     if (r[NSP - 1] < 0) r[NSP - 1] = 0.0;  // N2: no increment, clipped as the others
-    E += dei;
+    E = fma(P.Ru, dei, E);
 }
 
 // Species clip and rescale to the mixture density of one cell (Source/EBR.cpp:341-355),
@@ -261,7 +258,7 @@ __device__ __forceinline__ void cell_props(const double* x, long long ns, const 
     const double ei = x[4 * ns] - rho * (0.5 * (ux * ux + uy * uy + uz * uz));
 #pragma unroll
     for (int n = 0; n < NSP; ++n) r[n] = x[(5 + n) * ns];
-    *T = get_t_given_ey(ei, r, P.Ru);
+    *T = get_t_given_ey(ei, r, P);
     *p = ckpy(r, *T, P.Ru);
 #pragma unroll
     for (int n = 0; n < NSP; ++n) Y[n] = r[n] * rhoinv;
@@ -696,7 +693,7 @@ __device__ __forceinline__ void c2prim_real(const DevParm& P, const double* u, c
     q[QU] = ux;
     q[QV] = uy;
     q[QW] = uz;
-    const double T = get_t_given_ey(ei, rhoi, P.Ru);
+    const double T = get_t_given_ey(ei, rhoi, P);
     const double p = ckpy(rhoi, T, P.Ru);
     q[QT] = T;
     q[QPRES] = p;

@@ -25,8 +25,8 @@ __constant__ MechTables c_mech;
 //   gp       per range, for H2O, H, O, OH, HO2, H2O2: g/(RT) relative to the
 //            elements as H2 and O2, constant, T .. T^4, 1/T and ln T terms;
 //   nw       nu W_n for nu = 0 .. 4;
-//   hw       -HP_n Ru / W_n and a0w = A0_n / W_n;
-//   inv_ru, rs, inv_rs   1 / Ru, 1e6 Ru / Patm and its inverse.
+//   hpw      -HP_n / W_n and a0w = A0_n / W_n.
+// What depends on Ru and Patm is a context's own (DevParm): these tables are shared.
 struct MechDerived {
     double q3[2][NSP], q5[2][NSP];
     double g6[2][NSP], g12[2][NSP], g20[2][NSP];
@@ -37,8 +37,7 @@ struct MechDerived {
     double uw[2][6][NSP];
     double gp[2][NSP - 3][7];
     double nw[5][NSP];
-    double hw[NSP], a0w[NSP];
-    double inv_ru, rs, inv_rs;
+    double hpw[NSP], a0w[NSP];
     // enthalpy polynomials h/R = T (c0 + T (c1 + ...)) + c5 per range, and the
     // species-pair constants of the Wilke rule (j < k): (W_j / W_k)^(1/4),
     // 1 / sqrt(8 + 8 W_k / W_j), W_k / W_j
@@ -147,7 +146,8 @@ __device__ __forceinline__ double newton_reference_order(double ein, const doubl
 // the reference's order and both end on the same iterate.  The step's tests are
 // integer compares of |dt|'s bits (FP64 compares run on the FP64 pipe); a NaN passes
 // them as it passes the reference's.
-__device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, double Ru) {
+__device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, const DevParm& P) {
+    const double Ru = P.Ru;
     const int maxiter = 200;
     const double ein = e, tmin = 250, tmax = 3500;
     double smin = 0, smax = 0, As = 0;
@@ -160,7 +160,7 @@ __device__ __forceinline__ double get_t_given_ey(double e, const double* rhoi, d
     const double emin = smin * (Ru * tmin), emax = smax * (Ru * tmax);
     if (ein < emin) return tmin - (emin - ein) / ckcvbs(tmin, rhoi, Ru);
     if (ein > emax) return tmax - (emax - ein) / ckcvbs(tmax, rhoi, Ru);
-    const double es = ein * c_mder.inv_ru;  // e / Ru
+    const double es = ein * P.inv_ru;  // e / Ru
     double t1 = es * rcp_cubic(As);
     if (t1 < tmin || t1 > tmax) t1 = tmin + (tmax - tmin) / (emax - emin) * (ein - emin);
     const long long mag = 0x7fffffffffffffffLL;
@@ -385,7 +385,8 @@ __device__ __forceinline__ void eliminate(double (&U)[NRE][NRE + 1], double (&ip
 
 // The substep's increments x[n] of the partial densities from the concentrations
 // sc [mol/cm3] (n < NRE) and their sum over all species
-__device__ __forceinline__ void chem_increment(const double* sc, double mixture, double T, double dt, double* x) {
+__device__ __forceinline__ void chem_increment(const double* sc, double mixture, double T, double dt, const DevParm& P,
+                                               double* x) {
     double U[NRE][NRE + 1];
 #pragma unroll
     for (int a = 0; a < NRE; ++a)
@@ -393,8 +394,8 @@ __device__ __forceinline__ void chem_increment(const double* sc, double mixture,
         for (int b = 0; b <= NRE; ++b) U[a][b] = a == b ? 1.0 : 0.0;
     const double lnT = log(T);
     const double invT = rcp_cubic(T);
-    const double RsT = c_mder.rs * T;
-    const double iRsT = c_mder.inv_rs * invT;
+    const double RsT = P.rs * T;
+    const double iRsT = P.inv_rs * invT;
     double iE[NRE], z[NRE], inv[NRE];
     {
         const int h = T < 1000 ? 0 : 1;

@@ -72,6 +72,9 @@ DevParm make_dev_parm(const ocfd_parm& p) {
     d.twoThirds = p.twoThirds;
     d.Ru = p.Ru;
     d.Patm = p.Patm;
+    d.inv_ru = 1.0 / p.Ru;
+    d.rs = p.Ru / p.Patm * 1e6;
+    d.inv_rs = 1.0 / d.rs;
     double g = p.eos_gamma;
     d.sw_tmp1 = 1.0 / (2.0 * g);
     d.sw_tmp2 = 2.0 * (g - 1.0);
