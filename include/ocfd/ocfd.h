@@ -719,6 +719,12 @@ void ocfd_set_tma_staging(int32_t on);
  * reference. */
 ocfd_status ocfd_check_rcp_f64(const double* x, double* fast, double* ieee, int64_t n, void* stream);
 
+/* Test hook: thread `thread` (0 .. 511) of every CTA of the network's kernels gives up
+ * its tensor-core completion waits at once, so that they end with OCFD_TIMEOUT as if
+ * they had run out for that thread alone; -1 (the default) none.  No counterpart in
+ * the reference. */
+ocfd_status ocfd_check_mlp_late_thread(ocfd_mlp* mlp, int32_t thread);
+
 #ifdef __cplusplus
 }
 #endif

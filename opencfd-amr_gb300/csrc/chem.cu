@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(MLP_THREADS) k_chem_surrogate(MlpNet net, cons
                                bf16x2_bits(f[k + 4], f[k + 5]), bf16x2_bits(f[k + 6], f[k + 7]));
         }
         float out[16];
-        ok = mlp_tile<G>(sm, a0, group, tid, tbase + 128 * group, bar, phase, out, nullptr, nullptr, 0);
+        ok = mlp_tile<G>(net.late, sm, a0, group, tid, tbase + 128 * group, bar, phase, out, nullptr, nullptr, 0);
         if (!ok || !valid) continue;
         float dY[NSP];
 #pragma unroll

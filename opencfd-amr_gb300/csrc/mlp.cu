@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128) k_tc_gemm(const uint16_t* __restrict__ A,
                      ks > 0 ? 1u : 0u);
         mma_commit(bar);
     }
-    const bool ok = mbar_wait(bar, 0);
+    const bool ok = mbar_wait_all(bar, 0, 0, 128);
     fence_after_sync();
     if (!ok) {
         if (tid == 0) atomicOr(err, 1u);
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_forward(MlpNet net, const u
         }
         float out[16];
         // stash layout: block t of layer l at ((l * ntile + t) * 128 + row) * 128
-        ok = mlp_tile<G>(sm, a0, group, gt, tbase + 128 * group, bar, phase, out,
+        ok = mlp_tile<G>(net.late, sm, a0, group, gt, tbase + 128 * group, bar, phase, out,
                          Z ? Z + (long long)t * 128 * 128 : nullptr, H ? H + (long long)t * 128 * 128 : nullptr,
                          (long long)ntile * 128);
         if (ok && gt < 128)
@@ -145,8 +145,8 @@ constexpr int SD_A = 3 * 128 * 128 * 2 + 128 * 16 * 2;  // dZ_l, BF16
 constexpr int SD_BAR = SD_A + 128 * 128 * 2, SD_RED = SD_BAR + 16, SD_TOT = SD_RED + 4 * 4;
 __host__ __device__ constexpr int sd_w(int l) { return SD_W + (l - 1) * 128 * 128 * 2; }
 
-__global__ void __launch_bounds__(MLP_THREADS) k_mlp_bwd(const uint16_t* __restrict__ Wt, const float* __restrict__ Y,
-                                                         const float* __restrict__ T, const float* __restrict__ Z,
+__global__ void __launch_bounds__(MLP_THREADS) k_mlp_bwd(int late, const uint16_t* __restrict__ Wt,
+                                                         const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ Z,
                                                          float* dZ4, float* dZ, float* lossp, int ntile, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + SD_BAR);
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_bwd(const uint16_t* __restr
                              smem_desc(smem_u32(sm + sd_w(l) + ks * 128 * 32)), idesc, ks > 0 ? 1u : 0u);
                 mma_commit(bar);
             }
-            ok = mbar_wait(bar, phase);
+            ok = mbar_wait_all(bar, phase, 0, MLP_THREADS, mlp_wait_limit(late));
             phase ^= 1u;
             fence_after_sync();
             if (!ok) break;
@@ -320,7 +320,8 @@ __device__ __forceinline__ void stage_columns(unsigned char* dst, const uint16_t
     }
 }
 
-__global__ void __launch_bounds__(WG_THREADS) k_mlp_bwd_weight(const float* __restrict__ dZ4, const float* __restrict__ dZ,
+__global__ void __launch_bounds__(WG_THREADS) k_mlp_bwd_weight(int late, const float* __restrict__ dZ4,
+                                                               const float* __restrict__ dZ,
                                                                const uint16_t* __restrict__ Xb,
                                                                const uint16_t* __restrict__ H, long long M, float* partW,
                                                                float* partb, unsigned* err) {
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_mlp_bwd_weight(const float* __re
     if (tid < N)
         partb[(long long)blockIdx.x * BTOT + BOFF(l) + tid] =
             (red[tid] + red[N + tid]) + (red[2 * N + tid] + red[3 * N + tid]);
-    const bool ok = mbar_wait(bar, 0);
+    const bool ok = mbar_wait_all(bar, 0, 0, WG_THREADS, mlp_wait_limit(late));
     fence_after_sync();
     if (!ok) {
         if (tid == 0) atomicOr(err, 1u);
@@ -438,6 +439,7 @@ struct ocfd_mlp {
     uint16_t* Wt = nullptr;  // W_1 .. W_4 transposed, at the offsets of Wb
     float norm[2 * ocfd::MLP_IN + 3 * ocfd::MLP_OUT] = {};
     long long steps = 0;
+    int late = -1;  // MlpNet::late
     // training scratch (max_batch rows)
     uint16_t* Xb = nullptr;
     float* Y = nullptr;
@@ -462,6 +464,7 @@ MlpNet mlp_net(const ocfd_mlp* n);
 static MlpNet net_of(const ocfd_mlp* n) { return mlp_net(n); }
 MlpNet mlp_net(const ocfd_mlp* n) {
     MlpNet d{};
+    d.late = n->late;
     d.W = n->Wb;
     d.b = n->b32;
     for (int i = 0; i < MLP_IN; ++i) {
@@ -505,9 +508,10 @@ static ocfd_status mlp_forward(ocfd_mlp* n, const float* X, long long M, cudaStr
 static ocfd_status mlp_backward(ocfd_mlp* n, const float* T, long long M, cudaStream_t st, int& nblk) {
     const int ntile = (int)(M / 128);
     nblk = std::min(ntile, n->ctx->num_sms);
-    k_mlp_bwd<<<nblk, MLP_THREADS, SD_TOT, st>>>(n->Wt, n->Y, T, n->Z, n->dZ4, n->dZ, n->lossp, ntile, n->ctx->d_error);
-    k_mlp_bwd_weight<<<dim3((unsigned)(M / CHUNK), 5), WG_THREADS, SW_TOT, st>>>(n->dZ4, n->dZ, n->Xb, n->H, M, n->partW,
-                                                                              n->partb, n->ctx->d_error);
+    k_mlp_bwd<<<nblk, MLP_THREADS, SD_TOT, st>>>(n->late, n->Wt, n->Y, T, n->Z, n->dZ4, n->dZ, n->lossp, ntile,
+                                                 n->ctx->d_error);
+    k_mlp_bwd_weight<<<dim3((unsigned)(M / CHUNK), 5), WG_THREADS, SW_TOT, st>>>(n->late, n->dZ4, n->dZ, n->Xb, n->H, M,
+                                                                              n->partW, n->partb, n->ctx->d_error);
     return check_launch("MLP backward");
 }
 
@@ -644,6 +648,12 @@ static ocfd_status mlp_check_error(ocfd_mlp* n, cudaStream_t st, const char* who
         cudaMemsetAsync(n->ctx->d_error, 0, sizeof(uint32_t), st);
         return fail(OCFD_TIMEOUT, std::string(who) + ": a tensor-core completion wait ran out");
     }
+    return OCFD_OK;
+}
+
+ocfd_status ocfd_check_mlp_late_thread(ocfd_mlp* n, int32_t thread) {
+    if (!n || thread < -1 || thread >= MLP_THREADS) return fail(OCFD_BAD_ARG, "ocfd_check_mlp_late_thread");
+    n->late = thread;
     return OCFD_OK;
 }
 

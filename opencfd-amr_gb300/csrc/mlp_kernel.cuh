@@ -55,7 +55,12 @@ struct MlpNet {
     float in_mu[MLP_IN], in_isd[MLP_IN];     // feature normalisation: (x - mu) * isd
     float out_mu[MLP_OUT], out_sd[MLP_OUT];  // target scaling: y * sd + mu
     float out_scale[MLP_OUT];                // > 0: y is sign(r) log1p(|r| / scale) of the rate r
+    int late = -1;                           // thread of every CTA that gives up its waits at once (test hook), or -1
 };
+// polls of this thread's completion waits
+__device__ __forceinline__ uint32_t mlp_wait_limit(int late) {
+    return (int)threadIdx.x == late ? 0u : tc::kWaitLimit;
+}
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
 
@@ -109,10 +114,10 @@ __device__ __forceinline__ void group_sync(int group, int threads) {
 // [(gt / 128) 128 / G, (gt / 128 + 1) 128 / G) of every hidden layer; the output
 // layer's 16 columns go to the first warpgroup (out[]).  Hidden activations go to
 // `zs` / `hs` (FP32 pre-activations, BF16 activations; may be null).  Returns
-// false when an MMA completion wait ran out.
+// false - to all threads of the group - when an MMA completion wait ran out.
 template <int G>
-__device__ __forceinline__ bool mlp_tile(unsigned char* sm, unsigned char* a0, int group, int gt, uint32_t tbase,
-                                         uint64_t* bar, uint32_t& phase, float* out, float* zs, uint16_t* hs,
+__device__ __forceinline__ bool mlp_tile(int late, unsigned char* sm, unsigned char* a0, int group, int gt,
+                                         uint32_t tbase, uint64_t* bar, uint32_t& phase, float* out, float* zs, uint16_t* hs,
                                          long long ld) {
     static_assert(G == 2 || G == 4, "warpgroups per tile");
     constexpr int CW = MLP_H / G;
@@ -134,7 +139,7 @@ __device__ __forceinline__ bool mlp_tile(unsigned char* sm, unsigned char* a0, i
                          idesc, ks > 0 ? 1u : 0u);
             mma_commit(bar);
         }
-        const bool ok = mbar_wait(bar, phase);
+        const bool ok = mbar_wait_all(bar, phase, group + 1, 128 * G, mlp_wait_limit(late));
         phase ^= 1u;
         fence_after_sync();
         if (!ok) return false;

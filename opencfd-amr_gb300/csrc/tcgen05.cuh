@@ -66,12 +66,30 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 }
 // bounded wait (non-blocking polls with a short sleep, well under a second in
 // all): false when the phase did not complete
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 22)) {
+constexpr uint32_t kWaitLimit = 1u << 22;
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = kWaitLimit) {
     for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_test_wait(bar, parity)) return true;
         if (i > 64) __nanosleep(32);
     }
     return false;
+}
+// the same wait by all `threads` threads of a CTA's barrier `id` (whole warps; id 0
+// with the CTA's size is __syncthreads'), with one outcome for all of them: threads
+// start to poll at different times, and one that gave up alone would leave the others
+// at the next barrier for good.  When it ran out for any, what is in flight gets one
+// more bounded wait before the caller gives up its operands and TMEM.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, int id, int threads,
+                                              uint32_t limit = kWaitLimit) {
+    const uint32_t mine = mbar_wait(bar, parity, limit) ? 1u : 0u;
+    __syncwarp();
+    uint32_t all;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(all)
+                 : "r"(mine), "r"(id), "r"(threads)
+                 : "memory");
+    if (!all) mbar_wait(bar, parity);
+    return all != 0;
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, one 128 x N x 16 step, issued by one thread

@@ -21,6 +21,7 @@ declare("ocfd_mlp_set_params", ctypes.c_int, [_vp, _vp, _vp])
 declare("ocfd_mlp_forward", ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int64, _vp])
 declare("ocfd_mlp_train_step", ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int64, ctypes.c_float, ctypes.c_int32,
                                               _fp, _vp, _vp, _vp])
+declare("ocfd_check_mlp_late_thread", ctypes.c_int, [_vp, ctypes.c_int32])
 
 
 def _f(a):
