@@ -1418,8 +1418,8 @@ extern "C" ocfd_status ocfd_chem_cells_surrogate(ocfd_context* ctx, ocfd_mlp* ml
     if (!ctx || !mlp || !g || n <= 0 || !U) return fail(OCFD_BAD_ARG, "ocfd_chem_cells_surrogate");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // fallback counters and list (the cells' indices; a component stride of n) in
-    // the context's scratch pool
-    unsigned long long* tot = static_cast<unsigned long long*>(scratch(ctx, 16 + sizeof(long long) * (size_t)n));
+    // the pool of these calls
+    unsigned long long* tot = static_cast<unsigned long long*>(cells_scratch(ctx, 16 + sizeof(long long) * (size_t)n));
     if (!tot) return fail(OCFD_OUT_OF_MEMORY, "ocfd_chem_cells_surrogate");
     unsigned* cnt = reinterpret_cast<unsigned*>(tot + 1);
     long long* list = reinterpret_cast<long long*>(tot + 2);

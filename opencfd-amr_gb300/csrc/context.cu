@@ -46,19 +46,22 @@ bool covers_flag(const ocfd_flag4* a, const ocfd_box& bx, int grow) {
     return true;
 }
 
-void* scratch(ocfd_context* ctx, size_t bytes) {
-    if (bytes <= ctx->scratch_bytes) return ctx->scratch;
-    if (ctx->scratch) cudaFree(ctx->scratch);
-    ctx->scratch = nullptr;
-    ctx->scratch_bytes = 0;
+static void* grow(void*& p, size_t& have, size_t bytes) {
+    if (bytes <= have) return p;
+    if (p) cudaFree(p);
+    p = nullptr;
+    have = 0;
     size_t want = bytes + bytes / 4;
-    if (cudaMalloc(&ctx->scratch, want) != cudaSuccess) {
+    if (cudaMalloc(&p, want) != cudaSuccess) {
+        p = nullptr;
         cudaGetLastError();
         return nullptr;
     }
-    ctx->scratch_bytes = want;
-    return ctx->scratch;
+    have = want;
+    return p;
 }
+void* scratch(ocfd_context* ctx, size_t bytes) { return grow(ctx->scratch, ctx->scratch_bytes, bytes); }
+void* cells_scratch(ocfd_context* ctx, size_t bytes) { return grow(ctx->cells, ctx->cells_bytes, bytes); }
 
 DevParm make_dev_parm(const ocfd_parm& p) {
     DevParm d{};
@@ -189,6 +192,7 @@ ocfd_status ocfd_context_destroy(ocfd_context* ctx) {
     if (!ctx) return OCFD_OK;
     cudaSetDevice(ctx->device);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->cells) cudaFree(ctx->cells);
     if (ctx->d_error) cudaFree(ctx->d_error);
     delete ctx;
     return OCFD_OK;

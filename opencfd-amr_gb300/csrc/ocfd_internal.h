@@ -61,6 +61,8 @@ struct ocfd_context {
     uint32_t* d_error = nullptr;   // device error word
     void* scratch = nullptr;       // scratch pool owned by the context
     size_t scratch_bytes = 0;
+    void* cells = nullptr;         // lists of the 0D cells' calls
+    size_t cells_bytes = 0;
     int num_sms = 0;
     double* eb_static_scratch = nullptr;  // device address of the allocation-free variant's array
 };
@@ -78,6 +80,10 @@ bool covers_flag(const ocfd_flag4* a, const ocfd_box& bx, int grow);
 
 // Ensures the context scratch pool holds at least `bytes`; returns its pointer.
 void* scratch(ocfd_context* ctx, size_t bytes);
+// The same for the 0D cells' calls, which wait for their stream before they return: a
+// pool of their own, since a larger one must not free what a captured box call holds,
+// nor be written while a box call of another stream still runs.
+void* cells_scratch(ocfd_context* ctx, size_t bytes);
 
 // Looks up the device address of the allocation-free cut-cell entry point's
 // static array for ctx's device (which must be current); loads eb.cu's device
