@@ -863,7 +863,7 @@ __device__ __forceinline__ void chem_split(const ChemBoxArgs& B, int i, int j, i
     double tB = t1 * fma(t2, un, e.outer), tS = t1 * e.inner;
     if (e.sup) {
         tB += tS;
-        tS = 0.0;
+        tS = zero_of(tB);
     }
     const double tp = e.up ? tB : tS, tm = e.up ? tS : tB;
 #pragma unroll

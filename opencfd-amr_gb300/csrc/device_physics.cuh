@@ -268,6 +268,11 @@ __device__ __forceinline__ SplitSide split_side(double un, double c) {
     e.sup = (__double2hiint(e.inner) ^ __double2hiint(un)) >= 0;
     return e;
 }
+// 0, or not a number where x is not finite: the other side of a supersonic cell, whose
+// eigenvalues' positive or negative parts are zeros that the reference multiplies
+__device__ __forceinline__ double zero_of(double x) {
+    return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000 ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
+}
 template <int D>
 __device__ __forceinline__ void sw_split_d(double d, double u, double v, double w, double c, double t1, double t2,
                                            double hc, double gm1, double* fp, double* fm) {
@@ -287,7 +292,7 @@ __device__ __forceinline__ void sw_split_d(double d, double u, double v, double 
         rB = __dadd_rn(rB, rS);
         mB = __dadd_rn(mB, mS);
         eB = __dadd_rn(eB, eS);
-        rS = mS = eS = 0.0;
+        rS = mS = eS = zero_of(eB);  // eB holds every input
     }
     const auto put = [&](int n, double big, double small) {
         fp[n] = e.up ? big : small;
