@@ -22,7 +22,7 @@ namespace ocfd {
 
 void mech_builtin(MechTables* t);
 
-ocfd_status mech_upload(const ocfd_parm& p) {
+ocfd_status mech_upload(const ocfd_parm& p, double* hw) {
     MechTables t;
     mech_builtin(&t);
     auto fetch = [](double* dst, const double* src, size_t n) -> bool {
@@ -55,7 +55,7 @@ ocfd_status mech_upload(const ocfd_parm& p) {
         }
     for (int a = 0; a < NSP; ++a) {
         md.inv_mw[a] = 1.0 / t.mw[a];
-        md.hpw[a] = -t.HP[a] * md.inv_mw[a];
+        hw[a] = -t.HP[a] * p.Ru * md.inv_mw[a];
         md.a0w[a] = t.A0[a] * md.inv_mw[a];
         for (int k = 0; k < 5; ++k) md.nw[k][a] = k * t.mw[a];
         for (int h = 0; h < 2; ++h) {
@@ -140,10 +140,10 @@ __device__ __forceinline__ void chem_cell(const double* u, double& E, double* r,
     for (int n = 0; n < NRE; ++n) {
         const double v = r[n] + drho[n];
         r[n] = v < 0 ? 0.0 : v;
-        dei = fma(c_mder.hpw[n], drho[n], dei);
+        dei = fma(P.hw[n], drho[n], dei);
     }
     if (r[NSP - 1] < 0) r[NSP - 1] = 0.0;  // N2: no increment, clipped as the others
-    E = fma(P.Ru, dei, E);
+    E += dei;
 }
 
 // Species clip and rescale to the mixture density of one cell (Source/EBR.cpp:341-355),

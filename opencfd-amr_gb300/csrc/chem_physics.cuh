@@ -25,7 +25,7 @@ __constant__ MechTables c_mech;
 //   gp       per range, for H2O, H, O, OH, HO2, H2O2: g/(RT) relative to the
 //            elements as H2 and O2, constant, T .. T^4, 1/T and ln T terms;
 //   nw       nu W_n for nu = 0 .. 4;
-//   hpw      -HP_n / W_n and a0w = A0_n / W_n.
+//   a0w      A0_n / W_n.
 // What depends on Ru and Patm is a context's own (DevParm): these tables are shared.
 struct MechDerived {
     double q3[2][NSP], q5[2][NSP];
@@ -37,7 +37,7 @@ struct MechDerived {
     double uw[2][6][NSP];
     double gp[2][NSP - 3][7];
     double nw[5][NSP];
-    double hpw[NSP], a0w[NSP];
+    double a0w[NSP];
     // enthalpy polynomials h/R = T (c0 + T (c1 + ...)) + c5 per range, and the
     // species-pair constants of the Wilke rule (j < k): (W_j / W_k)^(1/4),
     // 1 / sqrt(8 + 8 W_k / W_j), W_k / W_j

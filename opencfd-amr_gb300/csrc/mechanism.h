@@ -25,7 +25,8 @@ void mech_builtin(MechTables* t);
 // reference's Source/Constants.cpp:15-150 data.
 void mech_host_tables(ocfd_parm* p);
 // Gathers the tables `p` points at (host or device memory; NULL members fall
-// back to the built-in data) and uploads them to constant memory.
-ocfd_status mech_upload(const ocfd_parm& p);
+// back to the built-in data) and uploads them to constant memory; hw receives
+// -HP_n Ru / W_n of the NSP species.
+ocfd_status mech_upload(const ocfd_parm& p, double* hw);
 
 }  // namespace ocfd

@@ -17,6 +17,7 @@ struct DevParm {
     double C_s, T_s, kOverMu, twoThirds;
     double Ru, Patm;
     double inv_ru, rs, inv_rs;         // 1/Ru, 1e6 Ru/Patm and its inverse: temperature inversion, reaction rates
+    double hw[OCFD_NSPEC];             // -HP_n Ru / W_n: the chemistry's energy per increment
     double sw_tmp1, sw_tmp2, sw_tmp3;  // 1/(2g), 2(g-1), (3-g)/(2(g-1)): FluxSplit.H:31-34
     double sw_gm1;                     // (g - 1) as written `(gamma - 1)` in FluxSplit.H:41
     double sw_hc;                      // 1/(g-1): the enthalpy's c^2 / (g - 1) of the fused FP64 split
