@@ -133,10 +133,10 @@ __global__ void k_mlp_pack(const float* __restrict__ X, uint16_t* Xb, long long 
 // routine's mirror image): the output gradient dZ_4 = dloss / dY of loss = mean over
 // rows and the 10 outputs of (Y - T)^2, then for l = 4..1 the product dZ_l W_l on the
 // tensor cores (A = dZ_l 128 x N_l, B(j, n) = W_l[n][j]) times gelu'(Z_{l-1}) in the
-// epilogue, which stores dZ_{l-1} in FP32 for the weight gradients and, as BF16, as
-// the next product's A operand.  The transposed weights of all four layers (100 KB)
-// are staged once per CTA; four warpgroups share a tile's epilogue by columns, which
-// bounds it (erf, exp).  A training step's batch of 8192 rows: four launches of one
+// epilogue, which stores dZ_{l-1} in FP32 in place of Z_{l-1} (nothing reads that any
+// more) for the weight gradients and, as BF16, as the next product's A operand.  The
+// transposed weights of all four layers (100 KB) are staged once per CTA; four
+// warpgroups share a tile's epilogue by columns, which bounds it (erf, exp).  A training step's batch of 8192 rows: four launches of one
 // warpgroup per tile, each staging its weights element by element, 164 us, this one
 // 36 us.
 // lossp[block] = the block's share of the sum of squares.
@@ -146,8 +146,8 @@ constexpr int SD_BAR = SD_A + 128 * 128 * 2, SD_RED = SD_BAR + 16, SD_TOT = SD_R
 __host__ __device__ constexpr int sd_w(int l) { return SD_W + (l - 1) * 128 * 128 * 2; }
 
 __global__ void __launch_bounds__(MLP_THREADS) k_mlp_bwd(int late, const uint16_t* __restrict__ Wt,
-                                                         const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ Z,
-                                                         float* dZ4, float* dZ, float* lossp, int ntile, unsigned* err) {
+                                                         const float* __restrict__ Y, const float* __restrict__ T,
+                                                         float* Z, float* dZ4, float* lossp, int ntile, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + SD_BAR);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + SD_BAR + 8);
@@ -226,17 +226,22 @@ __global__ void __launch_bounds__(MLP_THREADS) k_mlp_bwd(int late, const uint16_
             fence_after_sync();
             if (!ok) break;
             const long long q0 = (long long)(l - 1) * M * 128 + row * 128 + cg * 32;
-            float v[32];
+            float z[32], v[32];  // all of the row's Z before its first store
+#pragma unroll
+            for (int c = 0; c < 32; c += 4) {
+                const float4 q = *reinterpret_cast<const float4*>(Z + q0 + c);
+                z[c] = q.x;
+                z[c + 1] = q.y;
+                z[c + 2] = q.z;
+                z[c + 3] = q.w;
+            }
             tmem_ld32(trow + (uint32_t)(cg * 32), v);
 #pragma unroll
             for (int c = 0; c < 32; c += 8) {
-                const float4 za = *reinterpret_cast<const float4*>(Z + q0 + c);
-                const float4 zb = *reinterpret_cast<const float4*>(Z + q0 + c + 4);
-                const float z[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[c + i] *= gelu_grad(z[i]);
-                *reinterpret_cast<float4*>(dZ + q0 + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-                *reinterpret_cast<float4*>(dZ + q0 + c + 4) = make_float4(v[c + 4], v[c + 5], v[c + 6], v[c + 7]);
+                for (int i = 0; i < 8; ++i) v[c + i] *= gelu_grad(z[c + i]);
+                *reinterpret_cast<float4*>(Z + q0 + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                *reinterpret_cast<float4*>(Z + q0 + c + 4) = make_float4(v[c + 4], v[c + 5], v[c + 6], v[c + 7]);
                 if (l > 1)
                     *reinterpret_cast<uint4*>(sm + SD_A + kmajor_offset(lrow, cg * 32 + c, 128)) =
                         make_uint4(bf16x2_bits(v[c], v[c + 1]), bf16x2_bits(v[c + 2], v[c + 3]),
@@ -443,10 +448,9 @@ struct ocfd_mlp {
     // training scratch (max_batch rows)
     uint16_t* Xb = nullptr;
     float* Y = nullptr;
-    float* Z = nullptr;      // 4 x M x 128
+    float* Z = nullptr;      // 4 x M x 128: pre-activations, then their gradients
     uint16_t* H = nullptr;   // 4 x M x 128
     float* dZ4 = nullptr;    // M x 16
-    float* dZ = nullptr;     // 4 x M x 128
     float* partW = nullptr;  // nchunk x WTOT
     float* partb = nullptr;  // nchunk x BTOT
     float* lossp = nullptr;
@@ -508,9 +512,9 @@ static ocfd_status mlp_forward(ocfd_mlp* n, const float* X, long long M, cudaStr
 static ocfd_status mlp_backward(ocfd_mlp* n, const float* T, long long M, cudaStream_t st, int& nblk) {
     const int ntile = (int)(M / 128);
     nblk = std::min(ntile, n->ctx->num_sms);
-    k_mlp_bwd<<<nblk, MLP_THREADS, SD_TOT, st>>>(n->late, n->Wt, n->Y, T, n->Z, n->dZ4, n->dZ, n->lossp, ntile,
+    k_mlp_bwd<<<nblk, MLP_THREADS, SD_TOT, st>>>(n->late, n->Wt, n->Y, T, n->Z, n->dZ4, n->lossp, ntile,
                                                  n->ctx->d_error);
-    k_mlp_bwd_weight<<<dim3((unsigned)(M / CHUNK), 5), WG_THREADS, SW_TOT, st>>>(n->late, n->dZ4, n->dZ, n->Xb, n->H, M,
+    k_mlp_bwd_weight<<<dim3((unsigned)(M / CHUNK), 5), WG_THREADS, SW_TOT, st>>>(n->late, n->dZ4, n->Z, n->Xb, n->H, M,
                                                                               n->partW, n->partb, n->ctx->d_error);
     return check_launch("MLP backward");
 }
@@ -549,7 +553,6 @@ ocfd_status ocfd_mlp_create(ocfd_context* ctx, int32_t max_batch, uint64_t seed,
     al((void**)&n->Z, 4 * 4 * M * 128);
     al((void**)&n->H, 2 * 4 * M * 128);
     al((void**)&n->dZ4, 4 * M * 16);
-    al((void**)&n->dZ, 4 * 4 * M * 128);
     al((void**)&n->partW, 4 * nchunk * WTOT);
     al((void**)&n->partb, 4 * nchunk * BTOT);
     al((void**)&n->lossp, 4 * 1024);
@@ -594,7 +597,7 @@ ocfd_status ocfd_mlp_create(ocfd_context* ctx, int32_t max_batch, uint64_t seed,
 
 ocfd_status ocfd_mlp_destroy(ocfd_mlp* n) {
     if (!n) return OCFD_OK;
-    void* ps[] = {n->W32, n->b32, n->mW, n->vW, n->mb, n->vb, n->Wb, n->Wt, n->Xb, n->Y, n->Z, n->H, n->dZ4, n->dZ,
+    void* ps[] = {n->W32, n->b32, n->mW, n->vW, n->mb, n->vb, n->Wb, n->Wt, n->Xb, n->Y, n->Z, n->H, n->dZ4,
                   n->partW, n->partb, n->lossp, n->gW, n->gb};
     for (void* p : ps) cudaFree(p);
     if (n->host) cudaFreeHost(n->host);

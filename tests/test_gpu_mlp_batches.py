@@ -29,3 +29,17 @@ def test_mlp_gradients_by_batch(ctx, M):  # noqa: F811
         assert np.linalg.norm(gW[sl] - wW[sl]) < 5e-3 * np.linalg.norm(wW[sl]), l
         sb = slice(mo.BOFF[l], mo.BOFF[l] + mo.LN[l])
         assert np.linalg.norm(gb[sb] - wb[sb]) < 5e-3 * np.linalg.norm(wb[sb]), l
+
+
+def test_training_memory_per_row(ctx):  # noqa: F811
+    """Inputs 32, outputs and their gradients 64 each, pre-activations 2048 (their
+    gradients in place), activations 1024, weight and bias partials 1681 bytes a row."""
+    import torch
+    M = 1 << 17
+    make_mlp(ctx, max_batch=256, seed=1).close()  # the kernels' code
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    net = make_mlp(ctx, max_batch=M, seed=1)
+    used = free - torch.cuda.mem_get_info()[0]
+    net.close()
+    assert used <= 4913 * M + (48 << 20)  # allocations in 2 MB pages, the parameters
