@@ -713,6 +713,14 @@ ocfd_status ocfd_measure_ffma2_peak(double* fp32x2_gflops);
  * same results.  No counterpart in the reference. */
 void ocfd_set_tma_staging(int32_t on);
 
+/* Test hook: the inviscid FP32-flux right-hand side of one box (arguments as in
+ * ocfd_rhs_regular_box_f64, face fluxes included) with the tile shape `tile` (0 .. 8);
+ * *staged receives whether the tiles are staged by TMA, which 6 .. 8 are where the
+ * array's base, strides and x offset allow it.  No counterpart in the reference. */
+ocfd_status ocfd_check_rhs_f32_tile(ocfd_context* ctx, const ocfd_array4* S, const ocfd_array4* dSdt,
+                                    const ocfd_array4* flux, ocfd_box bx, const double dxinv[3], int32_t tile,
+                                    int32_t* staged, void* stream);
+
 /* Test hook: fast[i] = the reciprocal the fused FP64 kernels use in place of an
  * IEEE division (approximate seed + two Newton-Raphson steps), ieee[i] = 1/x[i]
  * correctly rounded; device arrays of n doubles.  No counterpart in the
