@@ -727,6 +727,12 @@ ocfd_status ocfd_check_rhs_f32_tile(ocfd_context* ctx, const ocfd_array4* S, con
  * reference. */
 ocfd_status ocfd_check_rcp_f64(const double* x, double* fast, double* ieee, int64_t n, void* stream);
 
+/* Test hook: the chemistry kernels' reciprocal (one cubic step from the approximate
+ * seed) and exponential (table-driven), and CUDA's exp, of x[i]; device arrays of n
+ * doubles.  No counterpart in the reference. */
+ocfd_status ocfd_check_chem_math_f64(const double* x, double* rcp, double* ex, double* cuda_exp, int64_t n,
+                                     void* stream);
+
 /* Test hook: thread `thread` (0 .. 511) of every CTA of the network's kernels gives up
  * its tensor-core completion waits at once, so that they end with OCFD_TIMEOUT as if
  * they had run out for that thread alone; -1 (the default) none.  No counterpart in

@@ -1438,3 +1438,24 @@ extern "C" ocfd_status ocfd_chem_cells_surrogate(ocfd_context* ctx, ocfd_mlp* ml
     if (fallbacks) *fallbacks = (int64_t)h;
     return s;
 }
+
+namespace ocfd {
+__global__ void k_chem_math_check(const double* __restrict__ x, double* __restrict__ rcp, double* __restrict__ ex,
+                                  double* __restrict__ cuda_exp, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        rcp[i] = rcp_cubic(x[i]);
+        ex[i] = exp_tab(x[i]);
+        cuda_exp[i] = exp(x[i]);
+    }
+}
+}  // namespace ocfd
+
+extern "C" ocfd_status ocfd_check_chem_math_f64(const double* x, double* rcp, double* ex, double* cuda_exp, int64_t n,
+                                                void* stream) {
+    if (!x || !rcp || !ex || !cuda_exp || n < 0) return ocfd::fail(OCFD_BAD_ARG, "ocfd_check_chem_math_f64");
+    if (n == 0) return OCFD_OK;
+    const long long blocks = (n + 255) / 256;
+    ocfd::k_chem_math_check<<<(int)(blocks < 4096 ? blocks : 4096), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        x, rcp, ex, cuda_exp, n);
+    return ocfd::check_launch("ocfd_check_chem_math_f64");
+}
