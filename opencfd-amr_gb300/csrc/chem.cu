@@ -49,9 +49,6 @@ ocfd_status mech_upload(const ocfd_parm& p, double* hw) {
             const double* a = h ? t.hi[n] : t.lo[n];
             md.q3[h][n] = a[2] / 3.0;
             md.q5[h][n] = a[4] / 5.0;
-            md.g6[h][n] = a[2] / 6.0;
-            md.g12[h][n] = a[3] / 12.0;
-            md.g20[h][n] = a[4] / 20.0;
         }
     for (int a = 0; a < NSP; ++a) {
         md.inv_mw[a] = 1.0 / t.mw[a];

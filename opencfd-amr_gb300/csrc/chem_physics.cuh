@@ -1,9 +1,11 @@
 // Li-Dryer H2/O2 thermochemistry and transport on the GPU (device functions).
 // Included by exactly one translation unit (chem.cu), which owns c_mech.
 //
-// Each routine keeps the operation order of the reference routine it replaces
-// (Source/CHEM/LiDryer.H, Source/CHEM/ChemViscous.H); exp/log/pow are CUDA's,
-// so results agree with the CPU build to a few ulps, not bit for bit.
+// The thermodynamic functions keep the operation order of the reference routines they
+// replace (Source/CHEM/LiDryer.H, Source/CHEM/ChemViscous.H).  The temperature
+// inversion, the reaction rates with their solution, and the transport coefficients are
+// regrouped, for the FP64 pipe, as said at each.  log and sqrt are CUDA's, exp in the
+// rates is exp_tab; results agree with the CPU build to a few ulps, not bit for bit.
 #pragma once
 
 #include "device_physics.cuh"
@@ -15,9 +17,8 @@ __constant__ MechTables c_mech;
 
 // Quantities derived from the tables once on the host, so that the per-cell
 // routines divide less (GB300's FP64 pipe runs a division as ~10 instructions):
-//   q3, q5   a2 / 3, a4 / 5 of the internal energy and enthalpy polynomials, and
-//   g6, g12, g20   a2 / 6, a3 / 12, a4 / 20 of the Gibbs polynomial - the same
-//            quotients the expressions form first, so these are bit-identical;
+//   q3, q5   a2 / 3, a4 / 5 of the internal energy and enthalpy polynomials - the
+//            same quotients the expressions form first, so these are bit-identical;
 //   inv_mw   1 / W_n, which replaces divisions by W (a rounding of the last bit
 //            differs from dividing);
 //   uw       per range, coefficient and species: the energy polynomial over W,
@@ -29,7 +30,6 @@ __constant__ MechTables c_mech;
 // What depends on Ru and Patm is a context's own (DevParm): these tables are shared.
 struct MechDerived {
     double q3[2][NSP], q5[2][NSP];
-    double g6[2][NSP], g12[2][NSP], g20[2][NSP];
     double inv_mw[NSP];
     // e_n(T)/(R T W_n) at the bounds 250 K and 3500 K of the temperature
     // inversion (the mixture energies there are then 9 products)
@@ -294,11 +294,10 @@ __device__ __forceinline__ double exp_tab(double x) {
 // cheaper.  Against the reference's expressions:
 //   - Equilibrium constants.  Every reaction conserves H and O, so Gibbs energies
 //     relative to H2 and O2, g'_n = g_n - (H_n / 2) g_H2 - (O_n / 2) g_O2, give
-//     the same reaction differences.  With E_n = (Ru T / Patm) exp_tab(g'_n) and
-//     z_n = c_n E_n, a reaction's rates are k' prod z (reactants) and k' prod z
+//     the same reaction differences.  With E_n = exp(g'_n) and z_n = c_n E_n, a
+//     reaction's rates are k' prod z (reactants) and (Ru T / Patm)^dn k' prod z
 //     (products), k' = k / prod E (reactants): six exponentials and reciprocals
-//     (g'_H2 = g'_O2 = 0) for the nineteen reactions, third-body factors
-//     (Ru T / Patm)^dn included.
+//     (g'_H2 = g'_O2 = 0) for the nineteen reactions.
 //   - d(rate)/dc_n = nu rate / (c_n + 1e-20): one reciprocal per species.
 //   - N2 takes part in no reaction: its row and column are the identity's, its
 //     increment is zero, and the system solved has the other eight species.
