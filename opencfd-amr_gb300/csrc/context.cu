@@ -67,8 +67,8 @@ DevParm make_dev_parm(const ocfd_parm& p) {
     DevParm d{};
     d.gamma = p.eos_gamma;
     d.Rg = p.Rg;
-    d.smallr = p.smallr;
-    d.smallp = p.smallp;
+    d.smallr = p.smallr + 0.0;  // a floor of -0 is 0: the kernels compare its bits
+    d.smallp = p.smallp + 0.0;
     d.C_s = p.C_s;
     d.T_s = p.T_s;
     d.kOverMu = p.kOverMu;
