@@ -678,7 +678,7 @@ def run_ours_jet(args, world, rank, local):
                                           "achieved_gbs": achieved32, "frac": achieved32 / hbm_peak,
                                           "ms_per_launch": reg_ms32, "achieved_gflops": flops32,
                                           "fp32_fma_peak_gflops": fp32.value,
-                                          "frac_of_fp32_fma_peak": flops32 / fp32.value}},
+                                          "reference_flops_over_fp32_peak": flops32 / fp32.value}},
                        "speedup_batched_over_per_box_fp64": (value / vpb) if vpb else None,
                        "finest_level_stage": fin_stage,
                        "kernels_per_coarse_step": {"fp64_batched": kernels / args.steps,
@@ -694,9 +694,10 @@ def run_ours_jet(args, world, rank, local):
                                    "(%d cells); the FP64 pipe, not HBM, binds it (see fp64)" % reg_cells,
                          "ms_per_launch": reg_ms, "alg_bytes_per_cell": 120,
                          "fp64": {"achieved_gflops": flops64, "peak_gflops": fp64.value,
-                                  "frac": flops64 / fp64.value,
+                                  # above 1: the kernel executes a fifth of the reference's operations
+                                  "reference_flops_over_peak": flops64 / fp64.value,
                                   "flops_per_cell_stage": FLOPS_PER_CELL_STAGE,
-                                  "counted": "the reference's formulation; the kernel executes about a fifth"},
+                                  "counted": "the reference's formulation"},
                          "fp32_fma_peak_gflops": fp32.value, "fp32x2_fma_peak_gflops": fp32x2.value},
             "cpu_baseline": cpu,
             "e2e": e2e64,

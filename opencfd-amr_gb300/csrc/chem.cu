@@ -827,13 +827,15 @@ __device__ __forceinline__ void visc_multi_face(const DevParm& P, const ChemBoxA
 //      FP32 (the mixed form; primitives narrowed on the integer pipes) per face;
 //   3. with viscosity, per face: Fick diffusion, viscous, heat and species-enthalpy
 //      fluxes (ChemViscous.H:108-355), in FP64, added to the fluxes of 2.
-// Bound by the FP64 pipe.  A thread per face that splits its own six stencil cells
-// does six times the splits and shares no differences between faces: 1590 FP64
-// instructions per face against 930 here.  8 lines x 24 faces take 52 KB of
+// Bound by the FP64 pipe (57 % busy) and the integer chain of the weights on 12 warps
+// per SM.  A thread per face that splits its own six stencil cells does six times the
+// splits and shares no differences between faces: 1590 FP64 instructions per face
+// against 930 in tiles when that was measured; with the correction in integers and the
+// split that places each eigenvalue once, 602.  8 lines x 24 faces take 52 KB of
 // shared memory (29 cells per line, odd: no bank conflicts along lines), 192 threads
 // one face each in 3; the three directions are one launch, so that a small box's
 // tiles fill the SMs (43x32x29 cells: 888 tiles).  Viscous box of 43x32x29 cells:
-// three directions 690 us a thread per face, 267 us here; in the mixed form, 32^3
+// three directions 690 us a thread per face, 227 us here; in the mixed form, 32^3
 // cells, 137 us and 82 us.
 constexpr int CF_LINES = 8, CF_FACES = 24, CF_CELLS = CF_FACES + 5, CF_THREADS = CF_LINES * CF_FACES;
 constexpr int CF_NC = 5 + NSP, CF_PLANE = CF_LINES * CF_CELLS;

@@ -305,9 +305,9 @@ __device__ __forceinline__ double exp_tab(double x) {
 //     Jacobian term is one FMA into the system's matrix.
 //   - Pivot search on the bits of |U| (integer), rows exchanged by selects,
 //     the pivot's reciprocal kept for the back substitution.
-// 6073 -> 1717 FP64 instructions per cell-substep, the FP64 pipe 88 % busy either
-// way: one substep of a 64^3 box 3025 -> 860 us, one step of a reacting 64^3 cube
-// (mixed form, 8 substeps) 30.6 -> 10.1 ms.  238-250 registers and no shared
+// 6073 -> 1678 FP64 instructions per cell-substep, the FP64 pipe 88 % busy either
+// way: one substep of a 64^3 box 3025 -> 840 us, one step of a reacting 64^3 cube
+// (mixed form, 8 substeps; with the faces and transport below) 30.6 -> 9.6 ms.  238-250 registers and no shared
 // memory (the 90-double matrix per thread was in shared memory): two CTAs of 128
 // threads per SM either way.
 constexpr int NRE = NSP - 1;  // reacting species (all but N2)
@@ -532,8 +532,8 @@ __device__ __forceinline__ double poly5(double x, const double* c) {
 // about 250 times per cell and take two square roots per species pair.  Here the
 // pair constants are tables, each species and each binary diffusivity has one
 // reciprocal, and each pair of the Wilke rule and of the diffusivities is visited
-// once, adding to both its species' sums: 4977 -> 1240 FP64 instructions per cell,
-// 685 -> 135 us on the 47430 cells around a 43x32x29 box, the FP64 pipe 88 % busy.
+// once, adding to both its species' sums: 4977 -> 1158 FP64 instructions per cell,
+// 685 -> 126 us on the 47430 cells around a 43x32x29 box, the FP64 pipe 87 % busy.
 __device__ __forceinline__ void transport(double T, double p, double rho, const double* r, double& mu, double& lambda,
                                           double* D) {
     double X[NSP], yow = 0.0;

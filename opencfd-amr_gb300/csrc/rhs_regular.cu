@@ -44,7 +44,10 @@ ocfd_status launch_rhs_regular(int tile, bool visc, const RegBoxArgs* d_boxes,
 // instructions; FP32: all), from its counts of work items per sweep: WENO-Z runs of
 // three faces x component (FP64) or faces x component (FP32), split cells of the
 // pencils, primitives (of the cross, or of each pencil and the ring with viscosity)
-// and viscous faces.  The weights are those of the kernels' instruction counts.
+// and viscous faces.  The weights are the kernels' instruction counts at the time the
+// tile shapes were measured (FP64 run 80, split 41; today's 60 and 27, and the integer
+// chain that runs beside them, are not in them): they rank the shapes, and the shapes
+// were measured with them.  The counts of today would choose otherwise for few sizes.
 static double tile_work(const TileShape& s, bool visc, bool f32) {
     const int T[3] = {s.x, s.y, s.z};
     auto warps = [](int items) { return (items + 31) / 32; };
@@ -71,6 +74,8 @@ static double tile_work(const TileShape& s, bool visc, bool f32) {
 //         tile's work for the last wave.  Tiles of which an SM holds two keep its
 //         FP64 pipe busier (one's barriers are the other's work), hence the factor.
 //   FP32  three and more tiles share an SM and overhanging ones do all their work.
+// The constants (0.5, 0.91, 0.35, 1.05 and the two rules of small shapes) are fitted to
+// the boxes below and some ten others of 20x12x8 to 128x96x64 cells.
 // Measured (us, the best shape of nine unless said; the rule takes these or is within
 // 3 %): FP64 viscous box of 20x12x8 cells 33 in 60 tiles of 4x4x2, 190 in six 8^3;
 // 13x97x5 45 in 8x2x2, 52 in 4x4x4; with the arithmetic before the split's and the

@@ -1,6 +1,7 @@
 // Fused regular-box right-hand side, templated on the precision of the flux
 // evaluation FT:
-//   FT = double  the plain FP64 form (reference operation order; parity 1e-12)
+//   FT = double  the plain FP64 form (split and WENO-Z regrouped for the FP64 pipe,
+//                the weights on the integer pipes; parity 1e-12)
 //   FT = float   the mixed-precision form: primitives, Steger-Warming split,
 //                WENO-Z (stencils normalised by a power of two, the smoothness
 //                epsilon rescaled into the normalised units), viscous flux and
@@ -14,7 +15,8 @@
 //      state, turned into primitives and split into F+ / F- (10 values per
 //      cell) in shared memory,
 //   2. WENO-Z face fluxes of the tile's T_D+1 faces x 5 components are formed
-//      in shared memory (work items = face x component),
+//      in shared memory (work items: FP32 face x component, FP64 a run of three
+//      faces x component, or in small tiles one side of a face x component),
 //   3. with OCFD_VISC the viscous stress / heat flux is added per face from a
 //      primitive ring (tile grown by 1) staged once per tile,
 //   4. each cell thread accumulates dxinv_D (F_f - F_f+1) in registers in the
